@@ -77,7 +77,8 @@ def draw(rng: random.Random):
     qtype = rng.choice(["q4_0", "q8_0", "f16"] if kind == "layer" else ["q4_0", "q8_0"])
     most = {"layer": 4096 if qtype == "f16" else 16384, "stack": 640, "host": 480, "step": 640}[kind]
     n = min(most, max(1, round(math.exp(rng.uniform(0.0, math.log(most))))))
-    return {"kind": kind, "qtype": qtype, "tokens": n, "routing": rng.choice(["even", "skewed", "zipf"])}
+    case = {"kind": kind, "qtype": qtype, "tokens": n, "routing": rng.choice(["even", "skewed", "zipf"])}
+    return case if all({**c, **case} != c for c in listed()) else draw(rng)
 
 
 # ------------------------------------------------------------------------------------------------------------- inputs
@@ -206,3 +207,74 @@ def tolerance(case):
     # Activations, SwiGLU products and outputs are fp16 (2^-11 a rounding, a handful of roundings to a layer), sums are f32.
     # Eleven layers add their roundings up, and a near-tie of the router may fall the other way in one of them.
     return {"rel": 2e-3 if case["kind"] == "layer" else 6e-3}
+
+
+# -------------------------------------------------------------------------------------------------------------- exact
+
+def _values(w: np.ndarray, s, qtype: str) -> torch.Tensor:
+    """The weights a model file's bytes stand for, flat, in 64 bits on the GPU."""
+    raw = torch.from_numpy(w).cuda()
+    if qtype == "f16":
+        return raw.view(torch.float16).double()
+    scale = torch.from_numpy(s.view(np.float16)).cuda().double().unsqueeze(1)
+    if qtype == "q8_0":
+        level = raw.view(torch.int8).double().reshape(-1, GROUP)
+    else:
+        raw = raw.reshape(-1, GROUP // 2)
+        level = torch.cat([raw & 15, raw >> 4], 1).double() - 8.0
+    return (level * scale).reshape(-1)
+
+
+def _swiglu(x, gate, up, down):
+    g = x @ gate.T
+    return (g * torch.sigmoid(g) * (x @ up.T)) @ down.T
+
+
+def _matrix_values(m, qtype: str) -> torch.Tensor:
+    return _values(m.qweight, m.qscale, qtype).reshape(m.rows, m.cols)
+
+
+def _moe(layer, qtype: str, x: torch.Tensor) -> torch.Tensor:
+    router = torch.from_numpy(layer.router.view(np.float16)).cuda().double().reshape(E, H)
+    logits = x @ router.T
+    if layer.logit_bias is not None:
+        logits += torch.from_numpy(layer.logit_bias).cuda().double()
+    probs, ids = torch.softmax(logits, 1).topk(K, 1)
+    out = _swiglu(x, _matrix_values(layer.shared_gate, qtype), _matrix_values(layer.shared_up, qtype),
+                  _matrix_values(layer.shared_down, qtype))
+    per_w, per_s = len(layer.expert_qweight) // E, 0 if layer.expert_qscale is None else len(layer.expert_qscale) // E
+    for e in ids.unique().tolist():
+        token, slot = (ids == e).nonzero(as_tuple=True)
+        scale = None if per_s == 0 else layer.expert_qscale[e * per_s:(e + 1) * per_s]
+        gate, up, down = _values(layer.expert_qweight[e * per_w:(e + 1) * per_w], scale, qtype).reshape(3, F * H)
+        y = _swiglu(x[token], gate.reshape(F, H), up.reshape(F, H), down.reshape(H, F))
+        out.index_add_(0, token, y * probs[token, slot].unsqueeze(1))
+    return out
+
+
+def exact(case, seed):
+    """What `run` returns, in 64 bits throughout (no rounding of activations); no value for the arg-max ids."""
+    kind, qtype, n = case["kind"], case["qtype"], case["tokens"]
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    rng = np.random.default_rng(seed)
+    layers = [_layer(gen, _routing_bias(rng, case["routing"]), qtype) for _ in range(1 if kind == "layer" else LAYERS)]
+    x = torch.randn((n, H), generator=gen, device="cuda").half().double()
+    if kind in ("stack", "host"):
+        for layer in layers:
+            x = x + _moe(layer, qtype, x)
+        return x
+    norms = [torch.rand(H, generator=gen, device="cuda").add_(0.5).half().double() for _ in range(LAYERS + 2)]
+
+    def normed(v, i):
+        return v / torch.sqrt(v.square().mean(1, keepdim=True) + EPS) * norms[i]
+
+    if kind == "layer":
+        return x + _moe(layers[0], qtype, normed(x, 0))
+    dense = [_matrix_values(_matrix(gen, *shape, qtype), qtype) for shape in ((DENSE, H), (DENSE, H), (H, DENSE))]
+    x = x + _swiglu(normed(x, 0), *dense)
+    for i, layer in enumerate(layers):
+        x = x + _moe(layer, qtype, normed(x, 1 + i))
+    out = normed(x, 1 + LAYERS)
+    heads = n if n <= 4 else 1
+    scores = out[n - heads:] @ _matrix_values(_matrix(gen, VOCAB, H, qtype), qtype).T
+    return out, None, scores.amax(1)
