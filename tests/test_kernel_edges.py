@@ -24,3 +24,26 @@ def test_fp16_grouped_gemm_honours_a_mixed_layer(pkg, port):
     """Quantised experts beside an fp16 shared MLP: both weight operands of the kernel in one call."""
     L, hidden, resid = make(41, dict(H=256, E=4, K=2, F=128, S=256), "q8_0", 70, shared_qname="f16")
     check_layer(pkg, port, L, hidden, resid, gemm=True)
+
+
+@pytest.mark.parametrize("n,K,E", [(31, 1, 8), (341, 3, 9), (512, 2, 8), (205, 5, 10), (1025, 1, 256), (1365, 6, 64), (1366, 6, 64)])
+def test_dispatch_plan_at_step_edges(pkg, n, K, E):
+    """Pair counts around a warp's step, a CTA's round and the limit of the one-CTA plan; some experts without pairs, some ids
+    out of range."""
+    rng = np.random.default_rng(n)
+    ids = rng.integers(0, max(1, E - 2), size=(n, K)).astype(np.uint32)
+    ids[rng.integers(0, n, 3), 0] = E + 1
+    off = torch.zeros(E + 1, dtype=torch.int32).cuda()
+    rows = torch.full((n * K,), -1, dtype=torch.int32).cuda()
+    inv = torch.zeros(n * K, dtype=torch.int32).cuda()
+    pkg.dispatch_plan_noalloc(dev(ids.view(np.int32)), n, K, E, off, rows, inv)
+    torch.cuda.synchronize()
+    flat = ids.reshape(-1)
+    order = np.argsort(flat, kind="stable")
+    order = order[flat[order] < E]
+    want_inv = np.full(n * K, 0xFFFFFFFF, dtype=np.uint32)
+    want_inv[order] = np.arange(order.size, dtype=np.uint32)
+    counts = np.bincount(flat[flat < E], minlength=E)
+    assert np.array_equal(off.cpu().numpy(), np.concatenate([[0], np.cumsum(counts)]))
+    assert np.array_equal(rows.cpu().numpy()[: order.size], order)
+    assert np.array_equal(inv.cpu().numpy().view(np.uint32), want_inv)

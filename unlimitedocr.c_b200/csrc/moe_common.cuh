@@ -186,6 +186,13 @@ struct SlicedKnobs {
 // Byte offsets inside the scratch region of the batched decode path.
 struct BatchedScratchLayout { size_t acc, x_limbs, x_scales, total; };
 
+// Where the tile lists of the routed grouped GEMMs go (gu null: none wanted), and how many weight-row tiles a token tile has.
+struct TileLists {
+    uint4 *gu, *dn;
+    uint32_t *counts;
+    uint32_t gu_mtiles, dn_mtiles;
+};
+
 // ---- launch interface (implemented in the kernel files, called by the host API) ----------
 struct LaunchCounter { uint64_t *count; };
 
@@ -194,7 +201,7 @@ cudaError_t launch_router(const DLayer &L, const __half *hidden, const float *in
                           cudaStream_t st, uint64_t *launches);
 cudaError_t launch_dispatch_plan(const uint32_t *ids, uint32_t n, uint32_t K, uint32_t E, uint32_t *offsets,
                                  uint32_t *pair_rows, uint32_t *inverse, uint32_t *active, uint32_t *chunk_counts,
-                                 cudaStream_t st, uint64_t *launches);
+                                 cudaStream_t st, uint64_t *launches, const TileLists &tiles = TileLists{});
 cudaError_t launch_small_batch_layer(const DLayer &L, const Scratch &S, const __half *hidden, const __half *residual,
                                      uint32_t n, __half *out, cudaStream_t st, uint64_t *launches);
 

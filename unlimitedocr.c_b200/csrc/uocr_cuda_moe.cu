@@ -34,7 +34,7 @@ cudaError_t init_gemm_kernels();
 bool gemm_path_supported(const DLayer &L);
 struct GemmScratch {
     __half *x_sorted, *mid_sorted, *down_sorted, *shared_mid, *shared_out;
-    uint4 *tiles_gu, *tiles_dn, *stiles_gu, *stiles_dn;
+    uint4 *tiles_gu, *tiles_dn;
     uint32_t *counts;
 };
 cudaError_t launch_scatter_peer(const DLayer &L, const Scratch &S, const __half *hidden, uint32_t n, uint32_t experts_per_rank,
@@ -55,7 +55,9 @@ cudaError_t launch_gather_sorted(const DLayer &L, const Scratch &S, const __half
                                  cudaStream_t st, uint64_t *launches);
 cudaError_t launch_gemm_experts(const DLayer &L, const Scratch &S, const GemmScratch &G, const uint32_t *seg_offsets,
                                 uint32_t n_seg, uint32_t expert_base, uint32_t expert_mod, const __half *rows_in,
-                                uint32_t rows_bound, __half *mid, __half *rows_out, cudaStream_t st, uint64_t *launches);
+                                uint32_t rows_bound, __half *mid, __half *rows_out, bool tiles_ready, cudaStream_t st,
+                                uint64_t *launches);
+TileLists gemm_tile_lists(const DLayer &L, const GemmScratch &G);
 cudaError_t launch_gemm_shared(const DLayer &L, const Scratch &S, const GemmScratch &G, const __half *hidden, uint32_t n,
                                cudaStream_t st, uint64_t *launches);
 cudaError_t launch_gemm_combine(const DLayer &L, const Scratch &S, const GemmScratch &G, const __half *down_rows,
@@ -118,8 +120,6 @@ struct uocr_cuda_context {
         uint32_t H = 0, S = 0, capacity = 0;
         __half *x_norm = nullptr, *mid = nullptr;      // [capacity][H], [capacity][S]
         float *out_f32 = nullptr;                      // [capacity][H] (the tensor-core path keeps fp16 rows in it)
-        uint4 *tiles_gu = nullptr, *tiles_dn = nullptr;
-        uint32_t *counts = nullptr;
         uint32_t units = 0;                            // one-token path through the decode kernel: 64-column units (0: not built)
         DLayer *d_layer = nullptr;                     // device copy of the pseudo layer that points at the units
         const uint8_t *unit_blobs = nullptr;
@@ -851,7 +851,7 @@ extern "C" int uocr_cuda_context_map_moe_layer(uocr_cuda_context *ctx, const uoc
 // ----------------------------------------------------------------------------------- arena
 struct ArenaLayout {
     uint64_t logits, probs, ids, weights, offsets, pair_rows, inverse, active, mid, shared_mid, down_out, shared_out,
-        stack0, stack1, d_in, d_res, d_out, dec_mid, dec_plogits, x_sorted, tiles_gu, tiles_dn, stiles_gu, stiles_dn,
+        stack0, stack1, d_in, d_res, d_out, dec_mid, dec_plogits, x_sorted, tiles_gu, tiles_dn,
         counts, plan_counts, seg_offsets, bt_routed, total;
 };
 
@@ -883,12 +883,10 @@ static ArenaLayout layout_arena(uint32_t H, uint32_t E, uint32_t K, uint32_t F, 
     a.dec_plogits = take((uint64_t)1024 * E * 4);           // and per-CTA partial router logits
     {   // tensor-core path: sorted activations and tile lists (a tile is 128 tokens x 128 rows of down, or x 64 rows each
         // of gate and up); the experts phase of an expert-parallel rank sees up to E segments
-        const uint64_t ttiles = (pairs + 127) / 128 + E, sttiles = ((uint64_t)n + 127) / 128;
+        const uint64_t ttiles = (pairs + 127) / 128 + E;
         a.x_sorted = take(pairs * H * 2);
         a.tiles_gu = take(ttiles * (F / 64 + 1) * 16);
         a.tiles_dn = take(ttiles * (H / 128 + 1) * 16);
-        a.stiles_gu = take(sttiles * (S / 64 + 1) * 16);
-        a.stiles_dn = take(sttiles * (H / 128 + 1) * 16);
         a.counts = take(64);
         a.seg_offsets = take(260 * 4);        // expert-parallel experts phase: offsets of the received segments
         a.plan_counts = take((pairs / 2048 + 2) * E * 4);
@@ -1062,7 +1060,6 @@ static uocr::GemmScratch gemm_scratch(uocr_cuda_context *ctx, const Scratch &s, 
     g.shared_mid = s.shared_mid;
     g.shared_out = (__half *)s.shared_out;
     g.tiles_gu = (uint4 *)(ctx->arena + a.tiles_gu); g.tiles_dn = (uint4 *)(ctx->arena + a.tiles_dn);
-    g.stiles_gu = (uint4 *)(ctx->arena + a.stiles_gu); g.stiles_dn = (uint4 *)(ctx->arena + a.stiles_dn);
     g.counts = (uint32_t *)(ctx->arena + a.counts);
     return g;
 }
@@ -1125,14 +1122,15 @@ static int layer_forward(uocr_cuda_context *ctx, uint32_t layer, const __half *d
         {
             ProfScope span(ctx, kPfPrefillPlan, ctx->stream);
             CU_TRY(ctx, uocr::launch_dispatch_plan(s.top_ids, n, L.K, L.E, s.expert_offsets, s.pair_rows, s.inverse,
-                                                   s.active, s.plan_counts, ctx->stream, &ctx->launches));
+                                                   s.active, s.plan_counts, ctx->stream, &ctx->launches,
+                                                   uocr::gemm_tile_lists(L, g)));
             CU_TRY(ctx, uocr::launch_gather_sorted(L, s, d_hidden, n, g.x_sorted, ctx->stream, &ctx->launches));
         }
         {
             ProfScope span(ctx, L.expert_qtype == UOCR_QT_Q4 ? kPfBucketedQ4 : (L.expert_qtype == UOCR_QT_Q8 ? kPfBucketedQ8 : kPfBucketedF16),
                            ctx->stream);
             CU_TRY(ctx, uocr::launch_gemm_experts(L, s, g, s.expert_offsets, L.E, 0, L.E, g.x_sorted, n * L.K, g.mid_sorted,
-                                                  g.down_sorted, ctx->stream, &ctx->launches));
+                                                  g.down_sorted, true, ctx->stream, &ctx->launches));
         }
         CU_TRY(ctx, cudaStreamWaitEvent(ctx->stream, ctx->join_event, 0));
         ProfScope span(ctx, kPfPrefillCombine, ctx->stream);
@@ -1229,17 +1227,14 @@ extern "C" int uocr_cuda_context_map_dense_mlp(uocr_cuda_context *ctx, const uoc
         if (sb && !upload(ctx, down->qscale, sb, &ps, error, error_size)) return 0;
         D.down = DMatrix{(const uint8_t *)pw, (const __half *)ps, H, S, (uint32_t)(wb / H), q};
     }
-    // scratch: normalised input, SwiGLU products, output rows, the two tile lists of the tensor-core path and their counts
+    // scratch: normalised input, SwiGLU products, output rows
     auto up256 = [](uint64_t v) { return (v + 255) & ~(uint64_t)255; };
-    const uint64_t token_tiles = (token_capacity + 127) / 128 + 1;
     const uint64_t o_x = 0, o_mid = o_x + up256((uint64_t)token_capacity * H * 2), o_out = o_mid + up256((uint64_t)token_capacity * S * 2),
-                   o_tg = o_out + up256((uint64_t)token_capacity * H * 4), o_td = o_tg + up256(token_tiles * (S / 64 + 1) * 16),
-                   o_cnt = o_td + up256(token_tiles * (H / 128 + 1) * 16), total = o_cnt + 256;
+                   total = o_out + up256((uint64_t)token_capacity * H * 4);
     uint8_t *base = nullptr;
     CU_TRY(ctx, cudaMalloc(&base, total));
     D.scratch = base; D.scratch_bytes = total;
     D.x_norm = (__half *)(base + o_x); D.mid = (__half *)(base + o_mid); D.out_f32 = (float *)(base + o_out);
-    D.tiles_gu = (uint4 *)(base + o_tg); D.tiles_dn = (uint4 *)(base + o_td); D.counts = (uint32_t *)(base + o_cnt);
     // One token: the single-token decode kernel on a slice-major copy of the three matrices (every CTA a 64-column unit)
     if (ctx->fused_decode && ctx->sliced_decode) {
         const uint32_t units = uocr::decode_dense_units(H, S, D.gate.qtype, D.up.qtype, D.down.qtype);
@@ -1281,8 +1276,7 @@ static int dense_forward(uocr_cuda_context *ctx, uint32_t index, const __half *d
         Scratch s{};
         s.status = ctx->status;
         uocr::GemmScratch g{};
-        g.shared_mid = D.mid; g.shared_out = (__half *)D.out_f32; g.stiles_gu = D.tiles_gu; g.stiles_dn = D.tiles_dn;
-        g.counts = D.counts - 2;                          // the shared MLP's two counters are entries 2 and 3
+        g.shared_mid = D.mid; g.shared_out = (__half *)D.out_f32;
         CU_TRY(ctx, uocr::launch_gemm_shared(L, s, g, d_hidden, n, ctx->stream, &ctx->launches));
         CU_TRY(ctx, uocr::launch_add_rows((const __half *)D.out_f32, d_residual, (size_t)n * D.H, d_out, ctx->stream, &ctx->launches));
         return 1;
@@ -1564,7 +1558,7 @@ extern "C" int uocr_cuda_moe_ep_experts(uocr_cuda_context *ctx, uint32_t layer, 
     CU_TRY(ctx, cudaEventRecord(ctx->seg_events[slot], ctx->stream));
     const uocr::GemmScratch g = gemm_scratch(ctx, s, a);
     CU_TRY(ctx, uocr::launch_gemm_experts(L, s, g, d_seg, n_seg, first_expert, n_local_experts,
-                                          (const __half *)d_rows_in, (uint32_t)run, g.mid_sorted, (__half *)d_rows_out,
+                                          (const __half *)d_rows_in, (uint32_t)run, g.mid_sorted, (__half *)d_rows_out, false,
                                           ctx->stream, &ctx->launches));
     return 1;
 }
@@ -1772,7 +1766,7 @@ extern "C" int uocr_cuda_moe_ep_peer_experts_dev(uocr_cuda_context *ctx, uint32_
     const unsigned long long cap_rows = (unsigned long long)ctx->token_capacity * L.K;
     const uint32_t bound = (uint32_t)(P.row_capacity < cap_rows ? P.row_capacity : cap_rows);      // rows this rank can hold
     CU_TRY(ctx, uocr::launch_gemm_experts(L, s, g, (const uint32_t *)(ctx->arena + a.seg_offsets), P.world * per, P.rank * per, per,
-                                          P.recv, bound, g.mid_sorted, P.done, ctx->stream, &ctx->launches));
+                                          P.recv, bound, g.mid_sorted, P.done, false, ctx->stream, &ctx->launches));
     return 1;
 }
 
@@ -1805,7 +1799,7 @@ extern "C" int uocr_cuda_moe_ep_peer_forward(uocr_cuda_context *ctx, uint32_t la
                                           ctx->stream, &ctx->launches));
     CU_TRY(ctx, uocr::launch_ep_signal_wait(P.sync, P.world, P.rank, 1, call, ctx->status, ctx->stream, &ctx->launches));
     CU_TRY(ctx, uocr::launch_gemm_experts(L, s, g, seg_offsets, P.world * per, P.rank * per, per, P.recv, (uint32_t)bound,
-                                          g.mid_sorted, P.done, ctx->stream, &ctx->launches));
+                                          g.mid_sorted, P.done, false, ctx->stream, &ctx->launches));
     CU_TRY(ctx, uocr::launch_ep_signal_wait(P.sync, P.world, P.rank, 2, call, ctx->status, ctx->stream, &ctx->launches));
     if (!join_shared(ctx, error, error_size)) return 0;
     CU_TRY(ctx, uocr::launch_combine_peer(L, s, g, P.done_all, per, P.d_dst_row0, P.row_capacity, (const __half *)d_residual, n,
