@@ -47,3 +47,33 @@ def test_dispatch_plan_at_step_edges(pkg, n, K, E):
     assert np.array_equal(off.cpu().numpy(), np.concatenate([[0], np.cumsum(counts)]))
     assert np.array_equal(rows.cpu().numpy()[: order.size], order)
     assert np.array_equal(inv.cpu().numpy().view(np.uint32), want_inv)
+
+
+@pytest.mark.parametrize("qname", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("n", [3, 4, 5, 16, 17])
+def test_batched_decode_at_n_block_edges(pkg, port, qname, n):
+    """Every token takes the same experts, so each item has n (or, above 16, 16 and n - 16) tokens: one to four blocks of four,
+    the first of which has its groups shared by two warps."""
+    L, hidden, resid = make(500 + n, FULL, qname, n)
+    hidden[:] = hidden[0]
+    check_layer(pkg, port, L, hidden, resid)
+
+
+@pytest.mark.parametrize("qname,n", [("q4_0", 2), ("q8_0", 5), ("q4_0", 64)])
+def test_batched_decode_with_the_norm_folded_in(pkg, qname, n):
+    """The routing kernel's own RMSNorm equals the norm kernel followed by the plain call bit for bit."""
+    L, hidden, _ = make(600 + n, FULL, qname, n)
+    w = torch.rand(FULL["H"], device="cuda").add_(0.5).half()
+    x = dev(hidden).view(torch.float16)
+    g = Layer(pkg, L, n)
+    try:
+        folded, normed, plain = (torch.zeros((n, FULL["H"]), dtype=torch.float16, device="cuda") for _ in range(3))
+        g.ctx.layer_forward_normed(0, x, w, 1e-6, n, folded)
+        g.ctx.rmsnorm(x, w, 1e-6, n, FULL["H"], normed)
+        g.ctx.layer_forward(0, normed, n, plain, residual=x)
+        g.ctx.synchronize()
+        assert torch.equal(folded, plain)
+        with pytest.raises(pkg.UocrCudaError, match="RMSNorm"):
+            g.ctx.layer_forward_normed(0, x, w, -1.0, n, folded)
+    finally:
+        g.close()

@@ -33,7 +33,7 @@
 namespace uocr {
 
 constexpr int kBtConsumers = 512;                              // 16 warps compute
-constexpr int kBtThreads = kBtConsumers + 32;                  // + one warp that issues the bulk copies
+constexpr int kBtThreads = kBtConsumers + 64;                  // + a warp that copies the weights, and one that copies the activations
 constexpr int kBtTokens = 16;                                  // tokens per pass
 // An item covers SLICES consecutive 64-wide slices of its expert (template parameter of the kernel): two for calls of more
 // than 16 tokens (7 parts per expert and pass), one for smaller calls (14 parts), whose ~150 two-slice items would leave most
@@ -54,6 +54,8 @@ constexpr int kRsThreads = 512;                                 // 16 warps: fou
 
 struct RouteSmallParams {
     const __half *hidden;           // [n][H]
+    const __half *norm_weight;      // optional fp16[H]: the layer's input is RMSNorm(hidden) * norm_weight
+    float norm_eps;
     const __half *router;           // [E][H]
     const float *bias;              // [E] or null
     const float *injected;          // [n][E] logits to use instead of the dot products, or null
@@ -85,6 +87,7 @@ __global__ void __launch_bounds__(kRsThreads) route_small_kernel(const RouteSmal
     for (int h = tid; h < H / 2; h += kRsThreads) reinterpret_cast<uint4 *>(prm.acc + (size_t)token * H)[h] = make_uint4(0u, 0u, 0u, 0u);
     if (tid < H / 8) reinterpret_cast<uint4 *>(s_x)[tid] = __ldg(reinterpret_cast<const uint4 *>(prm.hidden + (size_t)token * H) + tid);
     __syncthreads();
+    if (prm.norm_weight != nullptr) rmsnorm_row_shared<H, kRsThreads>(s_x, prm.norm_weight, prm.norm_eps, s_probs);
 
     if (prm.injected != nullptr) {
         if (tid < E) s_logits[tid] = prm.injected[(size_t)token * E + tid] + (prm.bias ? prm.bias[tid] : 0.f);
@@ -213,7 +216,6 @@ struct BatchedParams {
     const uint32_t *x_limbs;          // [n][20][2][16 words]
     const float *x_scales;            // [n][20]
     uint32_t n, K;
-    const uint32_t *active;           // [0] = number of experts with at least one pair, then their ids
     const uint32_t *expert_offsets;   // [E + 1]
     const uint32_t *pair_rows;        // pairs grouped by expert
     const float *top_weights;         // [n][K] routing weights
@@ -246,7 +248,10 @@ template <int QT> struct BtSmem {
     static constexpr int kWt = kTok + 64;                                   // routing weight of each slot of the pass [16]
     static constexpr int kEntry = kWt + 64;                                 // entries (expert ids), most tokens first [66]
     static constexpr int kFirst = kEntry + 68 * 4;                          // first (entry, pass) index of each entry [67]
-    static constexpr int kBars = kFirst + 68 * 4;                           // full[4], empty[4], sc_full[2], sc_empty[2], flags
+    static constexpr int kOff = kFirst + 68 * 4;                            // first pair of each expert [65]
+    static constexpr int kPairTok = kOff + 68 * 4;                          // token of each pair, in expert order
+    static constexpr int kPairWt = kPairTok + kBtMaxTokens * 16 * 4;        // its routing weight
+    static constexpr int kBars = kPairWt + kBtMaxTokens * 16 * 4;           // full[4], empty[4], sc_full[2], sc_empty[2], x_full, x_empty, flags
     static constexpr int kTotal = kBars + 128;
 };
 
@@ -288,56 +293,108 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
     uint32_t *s_entry = reinterpret_cast<uint32_t *>(smem + Sm::kEntry);
     uint32_t *s_first = reinterpret_cast<uint32_t *>(smem + Sm::kFirst);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + Sm::kBars), *empty = full + kBtStages, *sc_full = empty + kBtStages,
-             *sc_empty = sc_full + 2;
-    int *s_flag = reinterpret_cast<int *>(sc_empty + 2);
+             *sc_empty = sc_full + 2, *x_full = sc_empty + 2, *x_empty = x_full + 1;
+    int *s_flag = reinterpret_cast<int *>(x_empty + 1);
+    uint32_t *s_off = reinterpret_cast<uint32_t *>(smem + Sm::kOff), *s_ptok = reinterpret_cast<uint32_t *>(smem + Sm::kPairTok);
+    float *s_pwt = reinterpret_cast<float *>(smem + Sm::kPairWt);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const uint32_t n_active = prm.active[0];
-    const uint32_t n_entries = n_active + kBtSharedHalves;
-
     if (tid == 0) {
         for (int i = 0; i < kBtStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], kBtConsumers / 32); }
         for (int i = 0; i < 2; ++i) { mbar_init(&sc_full[i], 1); mbar_init(&sc_empty[i], kBtConsumers / 32); }
+        mbar_init(x_full, 1);
+        mbar_init(x_empty, kBtConsumers / 32);
         s_flag[0] = 1; s_flag[1] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // The whole dispatch plan goes to shared memory once (at most 1024 pairs): an item then starts without a chain of loads
+    // from global memory (plan -> pair -> token -> activations), which took 5400 of an item's 17400 cycles and during which
+    // the weight ring filled up and stalled.  With it, the norm folded into the routing kernel and the groups of small items
+    // shared between two warps, a Q8_0 call of 8 tokens takes 48 us (52 before), a Q4_0 call of 37 tokens 77 us (79).
+    if (tid <= kSlE) s_off[tid] = prm.expert_offsets[tid];
+    for (uint32_t i = tid; i < prm.n * prm.K; i += kBtThreads) {
+        const uint32_t pair = prm.pair_rows[i];               // (positions past the last valid pair are not read below)
+        if (pair < prm.n * prm.K) { s_ptok[i] = pair / prm.K; s_pwt[i] = prm.top_weights[pair]; }
+    }
+    __syncthreads();
     // the entries ordered by their number of tokens, most first (the shared halves lead: every token takes them; then
-    // the selected experts, ties by id): rank by counting
-    auto entry_count = [&](uint32_t e) { return e >= (uint32_t)kSlE ? prm.n : prm.expert_offsets[e + 1] - prm.expert_offsets[e]; };
-    if ((uint32_t)tid < n_entries) {
-        const uint32_t e = (uint32_t)tid < (uint32_t)kBtSharedHalves ? (uint32_t)kSlE + tid : prm.active[1 + tid - kBtSharedHalves];
-        const uint32_t c = entry_count(e);
-        uint32_t rank = 0;
-        for (uint32_t j = 0; j < n_entries; ++j) {
-            const uint32_t e2 = j < (uint32_t)kBtSharedHalves ? (uint32_t)kSlE + j : prm.active[1 + j - kBtSharedHalves];
-            const uint32_t c2 = entry_count(e2);
-            rank += (c2 > c || (c2 == c && (e2 >= (uint32_t)kSlE ? e2 - kSlE : e2 + kBtSharedHalves) < (e >= (uint32_t)kSlE ? e - kSlE : e + kBtSharedHalves))) ? 1u : 0u;
+    // the selected experts, ties by id): eight threads per entry count the entries before it
+    auto entry_count = [&](uint32_t e) { return e >= (uint32_t)kSlE ? prm.n : s_off[e + 1] - s_off[e]; };
+    uint32_t before = 0, mine = 0;
+    const uint32_t order = (uint32_t)tid >> 3;                // shared halves 0 and 1, then the experts
+    auto entry_of = [&](uint32_t o) { return o < (uint32_t)kBtSharedHalves ? (uint32_t)kSlE + o : o - kBtSharedHalves; };
+    if (order < (uint32_t)kBtEntries) {
+        mine = entry_count(entry_of(order));
+        for (uint32_t o = (uint32_t)tid & 7u; o < (uint32_t)kBtEntries; o += 8u) {
+            const uint32_t c = entry_count(entry_of(o));
+            before += (c > mine || (c == mine && o < order)) ? 1u : 0u;
         }
-        s_entry[rank] = e;
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (order < (uint32_t)kBtEntries && (tid & 7) == 0) s_entry[before] = entry_of(order);       // experts without pairs come last
+    __syncthreads();
+    if (warp == 0) {                                          // (entry, pass) items before each entry: lane l takes entries 3l .. 3l + 2
+        uint32_t passes[3], sum = 0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const uint32_t k = 3u * lane + i;
+            passes[i] = k < (uint32_t)kBtEntries ? (entry_count(s_entry[k]) + kBtTokens - 1) / kBtTokens : 0u;
+            sum += passes[i];
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        uint32_t run = incl - sum;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const uint32_t k = 3u * lane + i;
+            if (k <= (uint32_t)kBtEntries) s_first[k] = run;
+            run += passes[i];
+        }
     }
     __syncthreads();
-    if (tid == 0) {
-        uint32_t run = 0;
-        for (uint32_t k = 0; k < n_entries; ++k) { s_first[k] = run; run += (entry_count(s_entry[k]) + kBtTokens - 1) / kBtTokens; }
-        s_first[n_entries] = run;
-    }
-    __syncthreads();
-    const uint32_t n_items = s_first[n_entries] * kBtParts;
+    const uint32_t n_items = s_first[kBtEntries] * kBtParts;
     if (blockIdx.x >= n_items) return;
     auto resolve = [&](uint32_t item) {
         BtItem it;
         const uint32_t ep = item / kBtParts;
         it.part = item % kBtParts;
-        uint32_t k = 0;
-        while (s_first[k + 1] <= ep) ++k;
+        uint32_t k = 0, hi = kBtEntries;                      // the entry with s_first[k] <= ep < s_first[k + 1]
+        while (hi - k > 1u) {
+            const uint32_t mid = (k + hi) >> 1;
+            if (s_first[mid] <= ep) k = mid; else hi = mid;
+        }
         it.expert = s_entry[k];
         it.p0 = (ep - s_first[k]) * kBtTokens;
-        it.row0 = it.expert >= (uint32_t)kSlE ? 0u : prm.expert_offsets[it.expert];
+        it.row0 = it.expert >= (uint32_t)kSlE ? 0u : s_off[it.expert];
         it.T = min((uint32_t)kBtTokens, entry_count(it.expert) - it.p0);
         return it;
     };
 
+    if (warp == kBtConsumers / 32 + 1) {
+        // ---- activations: as soon as the consumers have finished the gate / up products of an item, lane t copies the
+        // bytes and scales of the next item's token t.  Slots beyond the item's tokens keep what they hold: a token is a
+        // column of the products of its own, and nothing reads those columns.
+        uint32_t done = 0;
+        for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x, ++done) {
+            const BtItem it = resolve(item);
+            if (done > 0u && !mbar_wait(x_empty, (done - 1u) & 1u, prm.status, s_flag)) return;
+            __syncwarp();
+            if (lane == 0) mbar_expect_tx(x_full, it.T * (uint32_t)(kBtTokenLimbBytes + kSlGroups * 4));
+            __syncwarp();
+            if ((uint32_t)lane < it.T) {
+                const uint32_t token = it.expert >= (uint32_t)kSlE ? it.p0 + lane : s_ptok[it.row0 + it.p0 + lane];
+                bulk_g2s(smem + Sm::kXf + lane * kBtTokenLimbBytes, prm.x_limbs + (size_t)token * (kBtTokenLimbBytes / 4), kBtTokenLimbBytes, x_full);
+                bulk_g2s(smem + Sm::kXs + lane * kSlGroups * 4, prm.x_scales + (size_t)token * kSlGroups, kSlGroups * 4, x_full);
+            }
+        }
+        return;
+    }
     if (warp == kBtConsumers / 32) {
         // ---- producer: the gate / up fragments of every (item, slice), chunk by chunk through the ring, and their scales
         if (lane == 0) {
@@ -376,7 +433,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
 
     // ---- consumers
     const int rb = warp & 7, nh = warp >> 3;       // gate / up: row block, and which n-blocks (nh, nh + 2) of the pass
-    uint32_t seq = 0, slices_done = 0;
+    uint32_t seq = 0, slices_done = 0, items_done = 0;
 #ifdef UOCR_BT_TRACE
     unsigned long long bt_local[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     BT_T0(bt_all);
@@ -386,43 +443,15 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
         const BtItem it = resolve(item);
         const bool shared = it.expert >= (uint32_t)kSlE;
         const uint32_t T = it.T, NB = (T + 3u) / 4u;
+        const bool single = NB == 1u;
         const uint32_t first_unit = it.expert * kSlRoutedPerSlot + it.part * kBtSlices;
-        if (tid < kBtTokens) {
-            uint32_t token = 0xffffffffu;
-            float wt = 0.f;
-            if ((uint32_t)tid < T) {
-                if (shared) { token = it.p0 + tid; wt = 1.0f; }
-                else {
-                    const uint32_t pair = prm.pair_rows[it.row0 + it.p0 + tid];
-                    token = pair / prm.K;
-                    wt = prm.top_weights[pair];
-                }
-            }
-            s_tok[tid] = token;
-            s_wt[tid] = wt;
+        if ((uint32_t)tid < T) {             // read after the barriers of the SwiGLU step below
+            s_tok[tid] = shared ? it.p0 + tid : s_ptok[it.row0 + it.p0 + tid];
+            s_wt[tid] = shared ? 1.0f : s_pwt[it.row0 + it.p0 + tid];
         }
-        bt_sync();
-        // 1. the pass's activation bytes and scales (slots beyond T: zeros), all loads of a thread in flight together
-        {
-            constexpr int kVecsPerToken = kBtTokenLimbBytes / 16;            // 160
-            constexpr int kPerThread = kBtTokens * kVecsPerToken / kBtConsumers;     // 5
-            uint4 v[kPerThread];
-#pragma unroll
-            for (int i = 0; i < kPerThread; ++i) {
-                const int idx = i * kBtConsumers + tid, tok = idx / kVecsPerToken, w = idx - tok * kVecsPerToken;
-                const uint32_t token = s_tok[tok];
-                v[i] = token != 0xffffffffu ? __ldg(reinterpret_cast<const uint4 *>(prm.x_limbs + (size_t)token * (kBtTokenLimbBytes / 4)) + w)
-                                            : make_uint4(0u, 0u, 0u, 0u);
-            }
-#pragma unroll
-            for (int i = 0; i < kPerThread; ++i) reinterpret_cast<uint4 *>(s_xf)[i * kBtConsumers + tid] = v[i];
-            if (tid < kBtTokens * kSlGroups) {
-                const int tok = tid / kSlGroups, Gi = tid - tok * kSlGroups;
-                const uint32_t token = s_tok[tok];
-                s_xs[tid] = token != 0xffffffffu ? prm.x_scales[(size_t)token * kSlGroups + Gi] : 0.f;
-            }
-        }
-        bt_sync();
+        bool got = mbar_wait(x_full, items_done & 1u, prm.status, s_flag);       // 1. the pass's activation bytes and scales
+        ++items_done;
+        __syncwarp();
         BT_ADD(0, bt_p1);
 #ifdef UOCR_BT_TRACE
         bt_local[8] += 1; bt_local[9] += T;
@@ -437,11 +466,11 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
             __half dslo[kBtBlocksPerWarp], dshi[kBtBlocksPerWarp];
             BT_ADD(1, bt_dw);
             BT_T0(bt_gu);
-            // 2. gate / up: rows 8 rb .. + 7 of both matrices x the tokens of n-blocks nh and nh + 2
+            // 2. gate / up: rows 8 rb .. + 7 of both matrices x the tokens of n-blocks nh and nh + 2; with a single n-block (up
+            // to four tokens) the two warps of a row block share the groups of every chunk instead
             float ag[2] = {0.f, 0.f}, au[2] = {0.f, 0.f};
             const __half *scg = s_sc + sb * (Bl::kGuScBytes / 2) + (8 * rb + g) * kSlGroups;
             const __half *scu = scg + 64 * kSlGroups;
-            bool got = true;
 #pragma unroll
             for (int c = 0; c < kBtChunks; ++c, ++seq) {
                 const uint32_t s = seq % kBtStages;
@@ -450,9 +479,10 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
                 if (c == 0) got = mbar_wait(&sc_full[sb], (slices_done >> 1) & 1u, prm.status, s_flag) && got;
                 BT_ADD(2, bt_w);
                 const uint4 *w4 = s_ring4 + (size_t)s * (Sm::kChunkBytes / 16);
-                if ((uint32_t)nh < NB) {
+                if ((uint32_t)nh < NB || single) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
+                        if (single && (q >> 1) != nh) continue;
                         const int Gi = 4 * c + q;
                         uint4 wa, wb;
                         if (QT == UOCR_QT_Q8) { wa = w4[((q * 8 + rb) * 2) * 32 + lane]; wb = w4[((q * 8 + rb) * 2 + 1) * 32 + lane]; }
@@ -460,7 +490,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
                         const float sg = __half2float(scg[Gi]), su = __half2float(scu[Gi]);
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
-                            const uint32_t nb = (uint32_t)nh + 2u * i;
+                            const uint32_t nb = (single ? 0u : (uint32_t)nh) + 2u * i;
                             if (nb < NB) {
                                 const int tokl = 4 * (int)nb + (g >> 1);
                                 const uint4 xb = *reinterpret_cast<const uint4 *>(s_xf + (((tokl * kSlGroups + Gi) * 2 + (g & 1)) * 4 + t) * 4);
@@ -478,7 +508,10 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
                 if (lane == 0) bt_arrive(&empty[s]);
             }
             __syncwarp();
-            if (lane == 0) bt_arrive(&sc_empty[sb]);
+            if (lane == 0) {
+                bt_arrive(&sc_empty[sb]);
+                if (sl == kBtSlices - 1) bt_arrive(x_empty);           // the activations have been read for the last time
+            }
             // the slice's `down` fragments arrive through the ring as three more chunks (32 blocks of 16 rows per chunk):
             // this warp's five blocks and their scales go to registers, and the stages are handed back at once
             {
@@ -508,6 +541,12 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
             BT_ADD(3, bt_gu);
             BT_T0(bt_sw);
             // 3. SwiGLU in registers: lane (g, t) holds gate and up of column 8 rb + g for token 4 nb + t
+            if (single) {                                              // the other warp's groups come through s_midf
+                float2 *part = reinterpret_cast<float2 *>(s_midf) + rb * 32 + lane;
+                if (nh == 1) *part = make_float2(ag[0], au[0]);
+                bt_sync();
+                if (nh == 0) { const float2 o = *part; ag[0] += o.x; au[0] += o.y; }
+            }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const uint32_t nb = (uint32_t)nh + 2u * i;
@@ -623,10 +662,11 @@ bool decode_batched_supported(const DLayer &L, uint32_t n) {
 // scratch: a region of decode_batched_scratch(n, K).total bytes; ticket: a word that is zero before the first call
 // (every call leaves it zero).
 cudaError_t launch_batched_route(const DLayer &L, const Scratch &S, const __half *hidden, const float *injected, uint32_t n,
-                                 float *logits, float *probs, uint8_t *scratch, uint32_t *ticket, cudaStream_t st, uint64_t *launches) {
+                                 float *logits, float *probs, uint8_t *scratch, uint32_t *ticket, cudaStream_t st, uint64_t *launches,
+                                 const __half *norm_weight, float norm_eps) {
     const BatchedScratchLayout lay = decode_batched_scratch(n, L.K);
     RouteSmallParams r{};
-    r.hidden = hidden; r.router = L.router; r.bias = L.bias; r.injected = injected; r.n = n; r.K = L.K; r.scaling = L.scaling;
+    r.hidden = hidden; r.norm_weight = norm_weight; r.norm_eps = norm_eps; r.router = L.router; r.bias = L.bias; r.injected = injected; r.n = n; r.K = L.K; r.scaling = L.scaling;
     r.logits_out = logits; r.probs_out = probs; r.ids = S.top_ids; r.weights = S.top_weights;
     r.x_limbs = reinterpret_cast<uint32_t *>(scratch + lay.x_limbs); r.x_scales = reinterpret_cast<float *>(scratch + lay.x_scales);
     r.offsets = S.expert_offsets; r.pair_rows = S.pair_rows; r.inverse = S.inverse; r.active = S.active;
@@ -652,7 +692,7 @@ cudaError_t launch_batched_experts(const DLayer &L, const Scratch &S, uint32_t n
     p.units = L.dec_units;
     p.x_limbs = reinterpret_cast<const uint32_t *>(scratch + lay.x_limbs); p.x_scales = reinterpret_cast<const float *>(scratch + lay.x_scales);
     p.n = n; p.K = L.K;
-    p.active = S.active; p.expert_offsets = S.expert_offsets; p.pair_rows = S.pair_rows;
+    p.expert_offsets = S.expert_offsets; p.pair_rows = S.pair_rows;
     p.top_weights = S.top_weights;
     p.acc = reinterpret_cast<unsigned long long *>(scratch + lay.acc);
     p.status = S.status;

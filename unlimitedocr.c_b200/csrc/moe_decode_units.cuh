@@ -113,5 +113,37 @@ __device__ __forceinline__ void load_word_values(const __half *group, int p, flo
     x[0] = f01.x; x[1] = f01.y; x[2] = f23.x; x[3] = f23.y;
 }
 
+// RMSNorm of one row of H fp16 values in shared memory, in place, with the arithmetic of rmsnorm_kernel (128 threads take
+// every 128th pair, a shuffle tree per warp, the four warp sums added in order): a kernel that normalises its input itself
+// equals the norm kernel followed by the plain kernel bit for bit.  All THREADS threads of the CTA call it, between
+// barriers; sums: four floats of shared memory.
+template <int H, int THREADS>
+__device__ __forceinline__ void rmsnorm_row_shared(__half *x, const __half *__restrict__ w, float eps, float *sums) {
+    const int tid = threadIdx.x;
+    __half2 *xw = reinterpret_cast<__half2 *>(x);
+    if (tid < 128) {
+        float ss = 0.f;
+        for (int i = tid; i < H / 2; i += 128) {
+            const float2 v = __half22float2(xw[i]);
+            ss = fmaf(v.x, v.x, ss);
+            ss = fmaf(v.y, v.y, ss);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if ((tid & 31) == 0) sums[tid >> 5] = ss;
+    }
+    __syncthreads();
+    float total = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) total += sums[i];
+    const float inv = 1.0f / sqrtf(total / (float)H + eps);
+    const __half2 *wr = reinterpret_cast<const __half2 *>(w);
+    __syncthreads();          // every thread has read the four sums before their place is used again
+    for (int i = tid; i < H / 2; i += THREADS) {
+        const float2 v = __half22float2(xw[i]), gw = __half22float2(wr[i]);
+        xw[i] = __floats2half2_rn(v.x * inv * gw.x, v.y * inv * gw.y);
+    }
+    __syncthreads();
+}
 
 }  // namespace uocr

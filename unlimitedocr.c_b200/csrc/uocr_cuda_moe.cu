@@ -67,7 +67,8 @@ uint32_t decode_batched_max_tokens();
 BatchedScratchLayout decode_batched_scratch(uint32_t n, uint32_t K);
 bool decode_batched_supported(const DLayer &L, uint32_t n);
 cudaError_t launch_batched_route(const DLayer &L, const Scratch &S, const __half *hidden, const float *injected, uint32_t n,
-                                 float *logits, float *probs, uint8_t *scratch, uint32_t *ticket, cudaStream_t st, uint64_t *launches);
+                                 float *logits, float *probs, uint8_t *scratch, uint32_t *ticket, cudaStream_t st, uint64_t *launches,
+                                 const __half *norm_weight, float norm_eps);
 cudaError_t launch_batched_experts(const DLayer &L, const Scratch &S, uint32_t n, uint8_t *scratch, cudaStream_t st, uint64_t *launches);
 cudaError_t launch_batched_combine(const DLayer &L, const Scratch &S, const __half *residual, uint32_t n, uint8_t *scratch, __half *out,
                                    cudaStream_t st, uint64_t *launches);
@@ -1064,8 +1065,8 @@ static uocr::GemmScratch gemm_scratch(uocr_cuda_context *ctx, const Scratch &s, 
     return g;
 }
 
-// norm_weight: only for a call that takes the single-token decode kernel (the caller checks): the kernel then normalises
-// d_hidden itself
+// norm_weight: only for a call that takes the single-token or the batched decode kernels (the caller checks): they then
+// normalise d_hidden themselves
 static int layer_forward(uocr_cuda_context *ctx, uint32_t layer, const __half *d_hidden, const __half *d_residual,
                          const float *d_injected, uint32_t n, __half *d_out, const uocr_cuda_moe_debug_outputs *dbg,
                          char *error, size_t error_size, const __half *norm_weight = nullptr, float norm_eps = 0.f) {
@@ -1095,7 +1096,7 @@ static int layer_forward(uocr_cuda_context *ctx, uint32_t layer, const __half *d
         {
             ProfScope span(ctx, kPfRouter, ctx->stream);
             CU_TRY(ctx, uocr::launch_batched_route(L, s, d_hidden, d_injected, n, logits, probs, scratch, batched_ticket(ctx), ctx->stream,
-                                                   &ctx->launches));
+                                                   &ctx->launches, norm_weight, norm_eps));
         }
         {
             ProfScope span(ctx, kPfRouted, ctx->stream);
@@ -1171,11 +1172,12 @@ extern "C" int uocr_cuda_moe_layer_forward_normed(uocr_cuda_context *ctx, uint32
     if (!check_call(ctx, layer, n, error, error_size)) return 0;
     if (!d_stream || !d_norm_weight_f16 || !d_out) return fail(ctx, error, error_size, "null argument");
     const DLayer &L = ctx->layers[layer];
-    if (n == 1 && ctx->fused_decode && ctx->sliced_decode && uocr::decode_sliced_supported(ctx->layers.data(), layer, 1)) {
-        // one token: the decode kernel normalises its input itself (same arithmetic as the norm kernel), one launch
+    if ((n == 1 && ctx->fused_decode && ctx->sliced_decode && uocr::decode_sliced_supported(ctx->layers.data(), layer, 1)) ||
+        (n >= 2 && ctx->batched_decode && uocr::decode_batched_supported(L, n))) {
+        // the decode kernels normalise their input themselves (same arithmetic as the norm kernel): one launch less
         if (!(eps >= 0.f)) return fail(ctx, error, error_size, "RMSNorm: eps must not be negative");
         CU_TRY(ctx, cudaSetDevice(ctx->device));
-        return layer_forward(ctx, layer, (const __half *)d_stream, (const __half *)d_stream, nullptr, 1, (__half *)d_out, dbg, error,
+        return layer_forward(ctx, layer, (const __half *)d_stream, (const __half *)d_stream, nullptr, n, (__half *)d_out, dbg, error,
                              error_size, (const __half *)d_norm_weight_f16, eps);
     }
     ArenaLayout a;
