@@ -36,7 +36,7 @@ def test_dispatch_plan_at_step_edges(pkg, n, K, E):
     off = torch.zeros(E + 1, dtype=torch.int32).cuda()
     rows = torch.full((n * K,), -1, dtype=torch.int32).cuda()
     inv = torch.zeros(n * K, dtype=torch.int32).cuda()
-    pkg.dispatch_plan_noalloc(dev(ids.view(np.int32)), n, K, E, off, rows, inv)
+    pkg.ffi.dispatch_plan_noalloc(dev(ids.view(np.int32)), n, K, E, off, rows, inv)
     torch.cuda.synchronize()
     flat = ids.reshape(-1)
     order = np.argsort(flat, kind="stable")
@@ -75,5 +75,25 @@ def test_batched_decode_with_the_norm_folded_in(pkg, qname, n):
         assert torch.equal(folded, plain)
         with pytest.raises(pkg.UocrCudaError, match="RMSNorm"):
             g.ctx.layer_forward_normed(0, x, w, -1.0, n, folded)
+    finally:
+        g.close()
+
+
+@pytest.mark.parametrize("qname,dims,n", [("f16", FULL, 2), ("f16", FULL, 3), ("f16", dict(H=2048, E=6, K=3, F=64, S=192), 9),
+                                          ("q4_0", dict(H=192, E=5, K=2, F=64, S=320), 5), ("q8_0", dict(H=2048, E=5, K=2, F=192, S=64), 7)])
+def test_matrix_vector_kernels_at_row_and_token_edges(pkg, port, qname, dims, n):
+    """One, two, up to four and more tokens per expert, rows shorter than a warp's step and as long as the staging buffer, and
+    activation rows that start at an address that is a multiple of two only."""
+    L, hidden, resid = make(700 + n, dims, qname, n)
+    check_layer(pkg, port, L, hidden, resid)
+    g = Layer(pkg, L, n)
+    try:
+        odd = torch.zeros(n * dims["H"] + 1, dtype=torch.float16, device="cuda")[1:]
+        odd.copy_(dev(hidden).view(torch.float16).reshape(-1))
+        outs = [torch.zeros((n, dims["H"]), dtype=torch.float16, device="cuda") for _ in range(2)]
+        g.ctx.layer_forward(0, dev(hidden).view(torch.float16), n, outs[0])
+        g.ctx.layer_forward(0, odd, n, outs[1])
+        g.ctx.synchronize()
+        assert torch.equal(outs[0], outs[1])
     finally:
         g.close()

@@ -6,7 +6,7 @@
 //
 // Work is grouped per selected expert (dispatch plan), so a weight row is read once per step for
 // all tokens routed to that expert; activations of up to four tokens at a time sit in shared
-// memory as f32.
+// memory as fp16.
 //
 //   gate_up : mid[pair][i]   = fp16( silu(gate_e[i].x) * (up_e[i].x) )     (routed and shared)
 //   down    : down_out[pair][h] = down_e[h] . mid[pair]                      (f32 scratch)
@@ -56,15 +56,105 @@ __device__ __forceinline__ bool resolve_group(const GroupSource &g, uint32_t gro
     return r.count != 0;
 }
 
+// Dot products of one packed row with M activation rows held as fp16 in shared memory.  What bounds these kernels is the
+// shared-memory reads of the activations: as f32, one value at a time, a 16-byte piece of an fp16 row cost 8 M reads with
+// eight-way bank conflicts; as fp16 it costs M 16-byte reads without any (two-way for Q8_0 and Q4_0, whose pieces are wider).
+// Values and the order of the additions are those of the f32 form (chunk_dot_q4 / _q8 / _f16), so results are the same bits.
+// One fp16 layer of 3 tokens (16 distinct experts, 128 MB of weights): 148 -> 99 us, all five kernels and the norm included.
+__device__ __forceinline__ void unpack8(const uint4 &v, float (&f)[8]) {
+    const __half2 *h = reinterpret_cast<const __half2 *>(&v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float2 t = __half22float2(h[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
+}
 template <int QT, int M>
-__device__ __forceinline__ void gate_up_rows(const uint8_t *gw, const __half *gs, const uint8_t *uw, const __half *us,
-                                             uint32_t cols, const float *xs, int lane, float (&g)[M], float (&u)[M]) {
+__device__ __forceinline__ void piece_dot(const uint4 &q, const __half *x, int ld, int c, float scale, float (&acc)[M]) {
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+    if constexpr (QT == UOCR_QT_F16) {
+        float wf[8];
+        unpack8(q, wf);
 #pragma unroll
-    for (int m = 0; m < M; ++m) { g[m] = 0.f; u[m] = 0.f; }
-    row_dot<QT, M>(gw, gs, cols, xs, (int)cols, lane, g);
-    row_dot<QT, M>(uw, us, cols, xs, (int)cols, lane, u);
+        for (int m = 0; m < M; ++m) {
+            float xf[8];
+            unpack8(*reinterpret_cast<const uint4 *>(x + m * ld + c * 8), xf);
 #pragma unroll
-    for (int m = 0; m < M; ++m) { g[m] = warp_sum(g[m]); u[m] = warp_sum(u[m]); }
+            for (int i = 0; i < 8; ++i) acc[m] = fmaf(wf[i], xf[i], acc[m]);
+        }
+    } else if constexpr (QT == UOCR_QT_Q8) {
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            float part = 0.f;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                float xf[8];
+                unpack8(*reinterpret_cast<const uint4 *>(x + m * ld + c * 16 + 8 * k), xf);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) part = fmaf((float)(int)(int8_t)((w[2 * k + i / 4] >> (8 * (i % 4))) & 0xffu), xf[i], part);
+            }
+            acc[m] = fmaf(part, scale, acc[m]);
+        }
+    } else {
+        const __half *xc = x + (c >> 1) * 64 + ((c & 1) << 4);
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            float part = 0.f;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                float xl[8], xh[8];
+                unpack8(*reinterpret_cast<const uint4 *>(xc + m * ld + 8 * k), xl);
+                unpack8(*reinterpret_cast<const uint4 *>(xc + m * ld + 32 + 8 * k), xh);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint32_t byte = (w[2 * k + i / 4] >> (8 * (i % 4))) & 0xffu;
+                    part = fmaf((float)((int)(byte & 15u) - 8), xl[i], part);
+                    part = fmaf((float)((int)(byte >> 4) - 8), xh[i], part);
+                }
+            }
+            acc[m] = fmaf(part, scale, acc[m]);
+        }
+    }
+}
+
+// A warp's weight row on its way to shared memory.  The copies are issued before the activations are staged (the row depends on
+// the expert only, the activations on a chain of three more loads) and all at once, so that a warp has its whole row (2.5 KB
+// of fp16 at 1280 columns) in flight; every lane later reads back the 16-byte pieces that it copied itself.  Pieces beyond
+// kStagePieces are read from global memory as they are needed.
+constexpr int kStagePieces = 256;                 // 4 KB
+__device__ __forceinline__ int staged_pieces(int pieces) { return pieces < kStagePieces ? pieces : kStagePieces; }
+__device__ __forceinline__ void stage_row(uint4 *stage, const uint8_t *wrow, int pieces, int lane) {
+    const int end = staged_pieces(pieces);
+    for (int c = lane; c < end; c += 32)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(stage + c)), "l"(wrow + (size_t)c * 16) : "memory");
+}
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <int QT, int M>
+__device__ __forceinline__ void row_dot_staged(const uint4 *stage, const uint8_t *wrow, const __half *srow, uint32_t cols, const __half *x,
+                                               int lane, float *out) {
+    constexpr int kPerGroup = UOCR_GROUP / ChunkTraits<QT>::kWeights;
+    const int pieces = (int)(cols / ChunkTraits<QT>::kWeights), staged = staged_pieces(pieces);
+    float acc[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) acc[m] = 0.f;
+#pragma unroll 2
+    for (int c = lane; c < pieces; c += 32) {
+        const uint4 q = c < staged ? stage[c] : __ldg(reinterpret_cast<const uint4 *>(wrow) + c);
+        piece_dot<QT, M>(q, x, (int)cols, c, QT == UOCR_QT_F16 ? 1.f : __half2float(srow[c / kPerGroup]), acc);
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) out[m] = warp_sum(acc[m]);
+}
+template <int QT>
+static size_t gemv_smem(uint32_t cols, uint32_t rows_per_warp) {
+    const uint32_t pieces = cols / ChunkTraits<QT>::kWeights;
+    return (size_t)kMaxM * cols * sizeof(__half) + (size_t)(pieces < (uint32_t)kStagePieces ? pieces : kStagePieces) * 16 * rows_per_warp * kGemvWarps;
+}
+// one row of fp16 activations into shared memory (cols: a multiple of 64; a caller's own rows may start at any even address)
+__device__ __forceinline__ void stage_activations(__half *xs, const __half *row, uint32_t cols) {
+    if (reinterpret_cast<uintptr_t>(row) & 15u) {
+        for (uint32_t k = threadIdx.x; k < cols; k += kGemvThreads) xs[k] = row[k];
+        return;
+    }
+    for (uint32_t k = threadIdx.x; k < cols / 8; k += kGemvThreads) reinterpret_cast<uint4 *>(xs)[k] = __ldg(reinterpret_cast<const uint4 *>(row) + k);
 }
 
 // grid.x covers the F (or S) output rows, one per warp; grid.y = group index.
@@ -74,40 +164,44 @@ gate_up_kernel(GroupSource src, const __half *__restrict__ hidden, uint32_t H, u
                const uint8_t *__restrict__ w_base, const __half *__restrict__ s_base, uint64_t expert_stride_bytes,
                uint64_t up_offset_bytes, uint64_t expert_scale_stride, uint64_t up_scale_offset, uint32_t row_bytes,
                __half *__restrict__ mid) {
-    extern __shared__ float xs[];   // [kMaxM][H]
+    extern __shared__ __align__(16) __half gemv_xs[];   // [kMaxM][H], then the warps' staged rows
+    __half *xs = gemv_xs;
     GroupRows rows;
     if (!resolve_group(src, blockIdx.y, rows)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t i = blockIdx.x * kGemvWarps + warp;          // output row
-    const uint32_t groups = H / UOCR_GROUP;
-    const uint8_t *gw = w_base + rows.expert * expert_stride_bytes + (size_t)i * row_bytes;
+    const uint32_t groups = H / UOCR_GROUP, row = min(i, F - 1u);
+    const uint8_t *gw = w_base + rows.expert * expert_stride_bytes + (size_t)row * row_bytes;
     const uint8_t *uw = gw + up_offset_bytes;
-    const __half *gs = s_base ? s_base + rows.expert * expert_scale_stride + (size_t)i * groups : nullptr;
+    const __half *gs = s_base ? s_base + rows.expert * expert_scale_stride + (size_t)row * groups : nullptr;
     const __half *us = s_base ? gs + up_scale_offset : nullptr;
+    const int pieces = (int)(H / ChunkTraits<QT>::kWeights);
+    uint4 *stage_g = reinterpret_cast<uint4 *>(xs + (size_t)kMaxM * H) + (size_t)warp * 2 * staged_pieces(pieces);
+    uint4 *stage_u = stage_g + staged_pieces(pieces);
+    stage_row(stage_g, gw, pieces, lane);
+    stage_row(stage_u, uw, pieces, lane);
 
     for (uint32_t r0 = 0; r0 < rows.count; r0 += kMaxM) {
         const uint32_t mc = min((uint32_t)kMaxM, rows.count - r0);
         __syncthreads();
-        for (uint32_t k = tid; k < mc * H; k += kGemvThreads) {
-            const uint32_t m = k / H, c = k - m * H;
+        for (uint32_t m = 0; m < mc; ++m) {
             const uint32_t pair = rows.pairs ? rows.pairs[r0 + m] : (r0 + m);
-            const uint32_t token = rows.pairs ? pair / src.K : pair;
-            xs[k] = __half2float(hidden[(size_t)token * H + c]);
+            stage_activations(xs + (size_t)m * H, hidden + (size_t)(rows.pairs ? pair / src.K : pair) * H, H);
         }
+        stage_wait();
         __syncthreads();
         if (i >= F) continue;
         float g[kMaxM], u[kMaxM];
         if (mc == 1) {
-            float g1[1], u1[1];
-            gate_up_rows<QT, 1>(gw, gs, uw, us, H, xs, lane, g1, u1);
-            g[0] = g1[0]; u[0] = u1[0];
+            row_dot_staged<QT, 1>(stage_g, gw, gs, H, xs, lane, g);
+            row_dot_staged<QT, 1>(stage_u, uw, us, H, xs, lane, u);
         } else if (mc == 2) {
-            float g2[2], u2[2];
-            gate_up_rows<QT, 2>(gw, gs, uw, us, H, xs, lane, g2, u2);
-            g[0] = g2[0]; u[0] = u2[0]; g[1] = g2[1]; u[1] = u2[1];
+            row_dot_staged<QT, 2>(stage_g, gw, gs, H, xs, lane, g);
+            row_dot_staged<QT, 2>(stage_u, uw, us, H, xs, lane, u);
         } else {
             // rows beyond mc read stale shared memory; their results are not stored
-            gate_up_rows<QT, kMaxM>(gw, gs, uw, us, H, xs, lane, g, u);
+            row_dot_staged<QT, kMaxM>(stage_g, gw, gs, H, xs, lane, g);
+            row_dot_staged<QT, kMaxM>(stage_u, uw, us, H, xs, lane, u);
         }
         if (lane == 0) {
             for (uint32_t m = 0; m < mc; ++m) {
@@ -124,41 +218,34 @@ __global__ void __launch_bounds__(kGemvThreads)
 down_kernel(GroupSource src, const __half *__restrict__ mid, uint32_t H, uint32_t F,
             const uint8_t *__restrict__ w_base, const __half *__restrict__ s_base, uint64_t expert_stride_bytes,
             uint64_t expert_scale_stride, uint32_t row_bytes, float *__restrict__ out) {
-    extern __shared__ float xs[];   // [kMaxM][F]
+    extern __shared__ __align__(16) __half gemv_xs[];   // [kMaxM][F], then the warps' staged rows
+    __half *xs = gemv_xs;
     GroupRows rows;
     if (!resolve_group(src, blockIdx.y, rows)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t h = blockIdx.x * kGemvWarps + warp;
     const uint32_t groups = F / UOCR_GROUP;
-    const uint8_t *dw = w_base + rows.expert * expert_stride_bytes + (size_t)h * row_bytes;
-    const __half *ds = s_base ? s_base + rows.expert * expert_scale_stride + (size_t)h * groups : nullptr;
+    const uint32_t wrow = min(h, H - 1u);
+    const uint8_t *dw = w_base + rows.expert * expert_stride_bytes + (size_t)wrow * row_bytes;
+    const __half *ds = s_base ? s_base + rows.expert * expert_scale_stride + (size_t)wrow * groups : nullptr;
+    const int pieces = (int)(F / ChunkTraits<QT>::kWeights);
+    uint4 *stage_d = reinterpret_cast<uint4 *>(xs + (size_t)kMaxM * F) + (size_t)warp * staged_pieces(pieces);
+    stage_row(stage_d, dw, pieces, lane);
 
     for (uint32_t r0 = 0; r0 < rows.count; r0 += kMaxM) {
         const uint32_t mc = min((uint32_t)kMaxM, rows.count - r0);
         __syncthreads();
-        for (uint32_t k = tid; k < mc * F; k += kGemvThreads) {
-            const uint32_t m = k / F, c = k - m * F;
+        for (uint32_t m = 0; m < mc; ++m) {
             const uint32_t row = rows.pairs ? rows.pairs[r0 + m] : (r0 + m);
-            xs[k] = __half2float(mid[(size_t)row * F + c]);
+            stage_activations(xs + (size_t)m * F, mid + (size_t)row * F, F);
         }
+        stage_wait();
         __syncthreads();
         if (h >= H) continue;
         float acc[kMaxM];
-#pragma unroll
-        for (int m = 0; m < kMaxM; ++m) acc[m] = 0.f;
-        if (mc == 1) {
-            float a1[1] = {0.f};
-            row_dot<QT, 1>(dw, ds, F, xs, (int)F, lane, a1);
-            acc[0] = a1[0];
-        } else if (mc == 2) {
-            float a2[2] = {0.f, 0.f};
-            row_dot<QT, 2>(dw, ds, F, xs, (int)F, lane, a2);
-            acc[0] = a2[0]; acc[1] = a2[1];
-        } else {
-            row_dot<QT, kMaxM>(dw, ds, F, xs, (int)F, lane, acc);
-        }
-#pragma unroll
-        for (int m = 0; m < kMaxM; ++m) acc[m] = warp_sum(acc[m]);
+        if (mc == 1) row_dot_staged<QT, 1>(stage_d, dw, ds, F, xs, lane, acc);
+        else if (mc == 2) row_dot_staged<QT, 2>(stage_d, dw, ds, F, xs, lane, acc);
+        else row_dot_staged<QT, kMaxM>(stage_d, dw, ds, F, xs, lane, acc);
         if (lane == 0)
             for (uint32_t m = 0; m < mc; ++m) {
                 const uint32_t row = rows.pairs ? rows.pairs[r0 + m] : (r0 + m);
@@ -194,7 +281,7 @@ static void launch_gate_up(const GroupSource &src, uint32_t n_groups, const __ha
                            const uint8_t *w, const __half *s, uint64_t stride, uint64_t up_off, uint64_t sstride,
                            uint64_t sup_off, uint32_t row_bytes, __half *mid, cudaStream_t st) {
     dim3 grid((F + kGemvWarps - 1) / kGemvWarps, n_groups);
-    gate_up_kernel<QT><<<grid, kGemvThreads, sizeof(float) * kMaxM * H, st>>>(src, hidden, H, F, w, s, stride, up_off,
+    gate_up_kernel<QT><<<grid, kGemvThreads, gemv_smem<QT>(H, 2), st>>>(src, hidden, H, F, w, s, stride, up_off,
                                                                               sstride, sup_off, row_bytes, mid);
 }
 
@@ -203,7 +290,7 @@ static void launch_down(const GroupSource &src, uint32_t n_groups, const __half 
                         const uint8_t *w, const __half *s, uint64_t stride, uint64_t sstride, uint32_t row_bytes,
                         float *out, cudaStream_t st) {
     dim3 grid((H + kGemvWarps - 1) / kGemvWarps, n_groups);
-    down_kernel<QT><<<grid, kGemvThreads, sizeof(float) * kMaxM * F, st>>>(src, mid, H, F, w, s, stride, sstride,
+    down_kernel<QT><<<grid, kGemvThreads, gemv_smem<QT>(F, 1), st>>>(src, mid, H, F, w, s, stride, sstride,
                                                                            row_bytes, out);
 }
 
@@ -219,11 +306,14 @@ static uint32_t packed_row_bytes(int qt, uint32_t cols) {
 }
 
 cudaError_t init_small_batch_kernels() {
-    // MoE layers stay below 48 KB of dynamic shared memory (4 rows x 2048 f32 = 32 KB); the dense MLP of the first
-    // decoder layer stages rows of its intermediate width (6848) for the down product: 4 x 8192 f32 = 128 KB
-    cudaError_t err = cudaFuncSetAttribute(down_kernel<UOCR_QT_Q4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmemBytes);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(down_kernel<UOCR_QT_Q8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmemBytes);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(down_kernel<UOCR_QT_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmemBytes);
+    // activations of four tokens in fp16 (gate/up: up to 3072 wide, down: the dense MLP's intermediate width, up to 8192) and
+    // the staged weight rows of eight warps (two rows each for gate/up), 4 KB a row at most
+    cudaError_t err = cudaSuccess;
+#define UOCR_GEMV_SMEM(QT)                                                                                                           \
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(gate_up_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 88 * 1024); \
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(down_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+    UOCR_GEMV_SMEM(UOCR_QT_Q4) UOCR_GEMV_SMEM(UOCR_QT_Q8) UOCR_GEMV_SMEM(UOCR_QT_F16)
+#undef UOCR_GEMV_SMEM
     return err;
 }
 
