@@ -52,11 +52,31 @@ def test_dispatch_plan_at_step_edges(pkg, n, K, E):
 @pytest.mark.parametrize("qname", ["q4_0", "q8_0"])
 @pytest.mark.parametrize("n", [3, 4, 5, 16, 17])
 def test_batched_decode_at_n_block_edges(pkg, port, qname, n):
-    """Every token takes the same experts, so each item has n (or, above 16, 16 and n - 16) tokens: one to four blocks of four,
-    the first of which has its groups shared by two warps."""
+    """Every token takes the same experts, so each item has n (or, above 16, 16 and n - 16) tokens: one to four blocks of four."""
     L, hidden, resid = make(500 + n, FULL, qname, n)
     hidden[:] = hidden[0]
     check_layer(pkg, port, L, hidden, resid)
+
+
+@pytest.mark.parametrize("qname", ["q4_0", "q8_0"])
+def test_batched_decode_gives_a_token_the_same_bits_in_every_batch(pkg, qname):
+    """64 tokens in one call and in calls of 2, 3, 4, 5, 16 and 17: their experts' items hold one to sixteen tokens, one slice or
+    two, and a sum in another order would show in some of the 81920 outputs."""
+    L, hidden, _ = make(550, FULL, qname, 64)
+    g = Layer(pkg, L, 64)
+    try:
+        x = dev(hidden).view(torch.float16)
+        whole, parts = (torch.zeros((64, FULL["H"]), dtype=torch.float16, device="cuda") for _ in range(2))
+        g.ctx.layer_forward(0, x, 64, whole)
+        for size in (2, 3, 4, 5, 16, 17):
+            parts.zero_()
+            last = 64 // size * size
+            for i in range(0, last, size):
+                g.ctx.layer_forward(0, x[i:i + size], size, parts[i:i + size])
+            g.ctx.synchronize()
+            assert torch.equal(whole[:last].view(torch.int16), parts[:last].view(torch.int16)), size
+    finally:
+        g.close()
 
 
 @pytest.mark.parametrize("qname,n", [("q4_0", 2), ("q8_0", 5), ("q4_0", 64)])

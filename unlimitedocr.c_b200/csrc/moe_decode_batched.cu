@@ -310,8 +310,8 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
     }
     // The whole dispatch plan goes to shared memory once (at most 1024 pairs): an item then starts without a chain of loads
     // from global memory (plan -> pair -> token -> activations), which took 5400 of an item's 17400 cycles and during which
-    // the weight ring filled up and stalled.  With it, the norm folded into the routing kernel and the groups of small items
-    // shared between two warps, a Q8_0 call of 8 tokens takes 48 us (52 before), a Q4_0 call of 37 tokens 77 us (79).
+    // the weight ring filled up and stalled.  With it and the norm folded into the routing kernel a Q8_0 call of 8 tokens takes
+    // 46 us (52 before), a Q4_0 call of 37 tokens 71 us (79), single passes with a cold L2.
     if (tid <= kSlE) s_off[tid] = prm.expert_offsets[tid];
     for (uint32_t i = tid; i < prm.n * prm.K; i += kBtThreads) {
         const uint32_t pair = prm.pair_rows[i];               // (positions past the last valid pair are not read below)
@@ -443,7 +443,6 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
         const BtItem it = resolve(item);
         const bool shared = it.expert >= (uint32_t)kSlE;
         const uint32_t T = it.T, NB = (T + 3u) / 4u;
-        const bool single = NB == 1u;
         const uint32_t first_unit = it.expert * kSlRoutedPerSlot + it.part * kBtSlices;
         if ((uint32_t)tid < T) {             // read after the barriers of the SwiGLU step below
             s_tok[tid] = shared ? it.p0 + tid : s_ptok[it.row0 + it.p0 + tid];
@@ -466,8 +465,10 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
             __half dslo[kBtBlocksPerWarp], dshi[kBtBlocksPerWarp];
             BT_ADD(1, bt_dw);
             BT_T0(bt_gu);
-            // 2. gate / up: rows 8 rb .. + 7 of both matrices x the tokens of n-blocks nh and nh + 2; with a single n-block (up
-            // to four tokens) the two warps of a row block share the groups of every chunk instead
+            // 2. gate / up: rows 8 rb .. + 7 of both matrices x the tokens of n-blocks nh and nh + 2.  One warp adds up all
+            // groups of a token in ascending order, whatever the item's token count: a token's result has the same bits in every
+            // batch.  (Two warps sharing the groups of an item of up to four tokens gave that up and cost time: 48 and 77 us
+            // where the calls above take 46 and 71.)
             float ag[2] = {0.f, 0.f}, au[2] = {0.f, 0.f};
             const __half *scg = s_sc + sb * (Bl::kGuScBytes / 2) + (8 * rb + g) * kSlGroups;
             const __half *scu = scg + 64 * kSlGroups;
@@ -479,10 +480,9 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
                 if (c == 0) got = mbar_wait(&sc_full[sb], (slices_done >> 1) & 1u, prm.status, s_flag) && got;
                 BT_ADD(2, bt_w);
                 const uint4 *w4 = s_ring4 + (size_t)s * (Sm::kChunkBytes / 16);
-                if ((uint32_t)nh < NB || single) {
+                if ((uint32_t)nh < NB) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        if (single && (q >> 1) != nh) continue;
                         const int Gi = 4 * c + q;
                         uint4 wa, wb;
                         if (QT == UOCR_QT_Q8) { wa = w4[((q * 8 + rb) * 2) * 32 + lane]; wb = w4[((q * 8 + rb) * 2 + 1) * 32 + lane]; }
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
                         const float sg = __half2float(scg[Gi]), su = __half2float(scu[Gi]);
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
-                            const uint32_t nb = (single ? 0u : (uint32_t)nh) + 2u * i;
+                            const uint32_t nb = (uint32_t)nh + 2u * i;
                             if (nb < NB) {
                                 const int tokl = 4 * (int)nb + (g >> 1);
                                 const uint4 xb = *reinterpret_cast<const uint4 *>(s_xf + (((tokl * kSlGroups + Gi) * 2 + (g & 1)) * 4 + t) * 4);
@@ -541,12 +541,6 @@ __global__ void __launch_bounds__(kBtThreads, 1) decode_batched_kernel(const __g
             BT_ADD(3, bt_gu);
             BT_T0(bt_sw);
             // 3. SwiGLU in registers: lane (g, t) holds gate and up of column 8 rb + g for token 4 nb + t
-            if (single) {                                              // the other warp's groups come through s_midf
-                float2 *part = reinterpret_cast<float2 *>(s_midf) + rb * 32 + lane;
-                if (nh == 1) *part = make_float2(ag[0], au[0]);
-                bt_sync();
-                if (nh == 0) { const float2 o = *part; ag[0] += o.x; au[0] += o.y; }
-            }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const uint32_t nb = (uint32_t)nh + 2u * i;
