@@ -242,7 +242,8 @@ UOCR_CUDA_API int uocr_cuda_rmsnorm(uocr_cuda_context *ctx, const void *d_x, con
 /* The MoE layer as the decoder runs it (src/backend/metal/uocr_metal.m:14433-14497): d_stream is the residual stream after
  * attention, the post-attention norm feeds the layer and the stream is added back:
  * d_out = MoE( RMSNorm(d_stream) * weight ) + d_stream.  The normalised rows live in the context's scratch; calls on
- * the single-token and the batched decode kernels normalise inside those (one launch less, the same arithmetic, bit-equal). */
+ * the single-token and the batched decode kernels normalise inside those (one launch less, the same arithmetic, bit-equal),
+ * the batched ones where d_stream starts at a multiple of 16 bytes. */
 UOCR_CUDA_API int uocr_cuda_moe_layer_forward_normed(uocr_cuda_context *ctx, uint32_t layer, const void *d_stream,
                                                      const void *d_norm_weight_f16, float eps, uint32_t n_tokens, void *d_out,
                                                      const uocr_cuda_moe_debug_outputs *dbg, char *error, size_t error_size);

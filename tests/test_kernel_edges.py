@@ -99,6 +99,32 @@ def test_batched_decode_with_the_norm_folded_in(pkg, qname, n):
         g.close()
 
 
+@pytest.mark.parametrize("qname,n", [("q4_0", 2), ("q8_0", 17), ("q4_0", 64)])
+def test_batched_decode_with_the_norm_on_a_stream_at_an_8_byte_address(pkg, qname, n):
+    """A stream that starts 8 bytes past a multiple of 16 takes the norm kernel (one launch more) and gives the same bits."""
+    L, hidden, _ = make(620 + n, FULL, qname, n)
+    w = torch.rand(FULL["H"], device="cuda").add_(0.5).half()
+    x = dev(hidden).view(torch.float16)
+    buf = torch.zeros(n * FULL["H"] + 8, dtype=torch.float16, device="cuda")
+    off = (8 - buf.data_ptr()) % 16 // 2
+    moved = buf[off:off + n * FULL["H"]].view(n, FULL["H"])
+    moved.copy_(x)
+    assert x.data_ptr() % 16 == 0 and moved.data_ptr() % 16 == 8
+    g = Layer(pkg, L, n)
+    try:
+        outs, launches = [], []
+        for rows in (x, moved):
+            out, before = torch.zeros((n, FULL["H"]), dtype=torch.float16, device="cuda"), g.ctx.kernel_launches
+            g.ctx.layer_forward_normed(0, rows, w, 1e-6, n, out)
+            g.ctx.synchronize()
+            outs.append(out)
+            launches.append(g.ctx.kernel_launches - before)
+        assert launches[1] == launches[0] + 1
+        assert torch.equal(outs[0], outs[1])
+    finally:
+        g.close()
+
+
 @pytest.mark.parametrize("qname,dims,n", [("f16", FULL, 2), ("f16", FULL, 3), ("f16", dict(H=2048, E=6, K=3, F=64, S=192), 9),
                                           ("q4_0", dict(H=192, E=5, K=2, F=64, S=320), 5), ("q8_0", dict(H=2048, E=5, K=2, F=192, S=64), 7)])
 def test_matrix_vector_kernels_at_row_and_token_edges(pkg, port, qname, dims, n):

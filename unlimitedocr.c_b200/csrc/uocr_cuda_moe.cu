@@ -1173,8 +1173,10 @@ extern "C" int uocr_cuda_moe_layer_forward_normed(uocr_cuda_context *ctx, uint32
     if (!d_stream || !d_norm_weight_f16 || !d_out) return fail(ctx, error, error_size, "null argument");
     const DLayer &L = ctx->layers[layer];
     if ((n == 1 && ctx->fused_decode && ctx->sliced_decode && uocr::decode_sliced_supported(ctx->layers.data(), layer, 1)) ||
-        (n >= 2 && ctx->batched_decode && uocr::decode_batched_supported(L, n))) {
-        // the decode kernels normalise their input themselves (same arithmetic as the norm kernel): one launch less
+        (n >= 2 && ctx->batched_decode && uocr::decode_batched_supported(L, n) && ((uintptr_t)d_stream & 15u) == 0)) {
+        // the decode kernels normalise their input themselves (same arithmetic as the norm kernel): one launch less.  The
+        // batched path's routing kernel reads rows in 16-byte loads, the norm kernel in 4-byte ones: a stream at any other
+        // address goes through the norm kernel, whose output rows are aligned (the single-token kernel reads two bytes at a time).
         if (!(eps >= 0.f)) return fail(ctx, error, error_size, "RMSNorm: eps must not be negative");
         CU_TRY(ctx, cudaSetDevice(ctx->device));
         return layer_forward(ctx, layer, (const __half *)d_stream, (const __half *)d_stream, nullptr, n, (__half *)d_out, dbg, error,
