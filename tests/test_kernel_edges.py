@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 from oracle import quant  # noqa: E402
-from test_cuda_moe import FULL, Layer, QT, check_layer, dev, make, pkg  # noqa: E402,F401
+from test_cuda_moe import FULL, Layer, QT, check_layer, dev, make, padded_slab_layer, pkg  # noqa: E402,F401
 
 
 @pytest.mark.parametrize("n,dims", [(16, dict(H=128, E=2, K=2, F=128, S=128)), (17, dict(H=256, E=3, K=1, F=128, S=384)),
@@ -24,6 +24,27 @@ def test_fp16_grouped_gemm_honours_a_mixed_layer(pkg, port):
     """Quantised experts beside an fp16 shared MLP: both weight operands of the kernel in one call."""
     L, hidden, resid = make(41, dict(H=256, E=4, K=2, F=128, S=256), "q8_0", 70, shared_qname="f16")
     check_layer(pkg, port, L, hidden, resid, gemm=True)
+
+
+@pytest.mark.parametrize("pad", [16, 48, 128 * 128 * 2])
+def test_fp16_slab_with_gaps_gives_the_packed_slabs_bits(pkg, pad):
+    """Gaps of any multiple of 16 bytes between the projections: strides that are no multiples of one another, and ones that are
+    multiples of a row but not of a matrix."""
+    L, hidden, _ = make(43, dict(H=128, E=4, K=2, F=256, S=128), "f16", 40)
+    outs, held = [], []
+    for layer in (L, padded_slab_layer(L, pad_bytes=pad)):
+        g = Layer(pkg, layer, 40)
+        try:
+            held.append(g.ctx.model_view_bytes)
+            for n in (1, 3, 40):
+                out = torch.zeros((n, L.H), dtype=torch.float16, device="cuda")
+                g.ctx.layer_forward(0, dev(hidden[:n]), n, out)
+                g.ctx.synchronize()
+                outs.append(out)
+        finally:
+            g.close()
+    assert held[0] == held[1]
+    assert all(torch.equal(a, b) for a, b in zip(outs[:3], outs[3:]))
 
 
 @pytest.mark.parametrize("n,K,E", [(31, 1, 8), (341, 3, 9), (512, 2, 8), (205, 5, 10), (1025, 1, 256), (1365, 6, 64), (1366, 6, 64)])

@@ -791,7 +791,19 @@ extern "C" int uocr_cuda_context_map_moe_layer(uocr_cuda_context *ctx, const uoc
         if (!upload(ctx, d->router_logit_bias, (uint64_t)E * 4, &p, error, error_size)) return 0;
         L.bias = (const float *)p;
     }
-    if (!upload(ctx, d->expert_qweight, (uint64_t)E * L.expert_stride_bytes, &p, error, error_size)) return 0;
+    if (qt == UOCR_QT_F16 && (L.expert_stride_bytes != 3 * proj || L.up_offset_bytes != proj || L.down_offset_bytes != 2 * proj)) {
+        // an fp16 slab with gaps is packed here: the tensor map that the grouped GEMM reads fp16 weights through wants strides
+        // that are multiples of one another
+        CU_TRY(ctx, cudaMalloc(&p, E * 3 * proj + kUploadPad));
+        ctx->weight_allocs.push_back(p);
+        CU_TRY(ctx, cudaMemset((uint8_t *)p + E * 3 * proj, 0, kUploadPad));
+        const uint64_t from[3] = {0, L.up_offset_bytes, L.down_offset_bytes};
+        for (int m = 0; m < 3; ++m)
+            CU_TRY(ctx, cudaMemcpy2D((uint8_t *)p + m * proj, 3 * proj, (const uint8_t *)d->expert_qweight + from[m], L.expert_stride_bytes, proj, E,
+                                     cudaMemcpyHostToDevice));
+        ctx->weight_bytes += E * 3 * proj;
+        L.expert_stride_bytes = 3 * proj; L.up_offset_bytes = proj; L.down_offset_bytes = 2 * proj;
+    } else if (!upload(ctx, d->expert_qweight, (uint64_t)E * L.expert_stride_bytes, &p, error, error_size)) return 0;
     L.expert_w = (const uint8_t *)p;
     if (qt != UOCR_QT_F16) {
         if (!upload(ctx, d->expert_qscale, (uint64_t)E * L.expert_scale_stride * 2, &p, error, error_size)) return 0;
