@@ -334,9 +334,11 @@ UOCR_CUDA_API int uocr_cuda_moe_dispatch_plan_noalloc(const uint32_t *d_top_ids,
  * dequantisers can be compared with the format definition (level * fp16 scale, src/model/uocr_format.h:49-99; the
  * reference pins its packed bytes in tests/test_convert.py:192-218 and unpacks them on the CPU only).
  *   matrix  0 / 1 / 2: gate [F][H] / up [F][H] / down [H][F] of routed expert `expert`; 3 / 4 / 5: the shared MLP's.
- *   path    0: the matrix-vector kernels (row_dot on one-hot activations): f32 level * float(scale), exact;
- *           1: the grouped GEMM's producer: fp16( float(level) * float(scale) ), the value the reference's tiled
- *              GEMMs feed their MMAs (src/backend/metal/kernels/gemm_q4.metal:35-57, gemm_q8.metal:43-60).
+ *   path    0: the matrix-vector kernels (their row product on one-hot activations): f32 level * float(scale), exact;
+ *           1: the grouped GEMM's weight operand: for Q4_0 / Q8_0 what its producer stores, fp16( float(level) * float(scale) ),
+ *              the value the reference's tiled GEMMs feed their MMAs (src/backend/metal/kernels/gemm_q4.metal:35-57,
+ *              gemm_q8.metal:43-60); for fp16, which the GEMM loads by TMA, the GEMM's product with one-hot rows (this
+ *              one allocates scratch and waits for the stream).
  * d_out: f32 [rows][cols] on the device.  path 1 needs cols to be a multiple of 64. */
 UOCR_CUDA_API int uocr_cuda_moe_debug_dequantize(uocr_cuda_context *ctx, uint32_t layer, uint32_t matrix, uint32_t expert,
                                                  uint32_t path, float *d_out, char *error, size_t error_size);

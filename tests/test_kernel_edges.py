@@ -26,6 +26,44 @@ def test_fp16_grouped_gemm_honours_a_mixed_layer(pkg, port):
     check_layer(pkg, port, L, hidden, resid, gemm=True)
 
 
+@pytest.mark.parametrize("hot", ["gate", "up", "down"])
+def test_fp16_grouped_gemm_reads_every_weight_from_its_place(pkg, hot):
+    """One-hot tokens through the GEMM's gate/up and down boxes, 128 to each of two experts and all 256 through the shared MLP:
+    output (token k, column h) is one weight of the matrix under test.  silu(64) = 64 and the other two matrices are constants or
+    (scaled) identities, so up and down come out exactly; gate as silu(w), a rounding to fp16 (2^-11) and the fast exponential away."""
+    D = 256
+    rng = np.random.default_rng(44)
+    eye, const = np.eye(D, dtype=np.float32), np.ones((D, D), dtype=np.float32)
+    # gate, up, down around the matrix w under test: out[k][h] = silu(w[h][k]), w[h][k], w[h][k]
+    others = {"gate": (None, const, eye), "up": (64 * const, None, eye), "down": (64 * const, eye / 64, None)}[hot]
+    tests = [rng.integers(-512, 512, (D, D)).astype(np.float32) / (8192 if hot == "up" else 128) for _ in range(3)]      # all fp16 values
+    full = [[w if m is None else m for m in others] for w in tests]
+    slab = np.concatenate([m.reshape(-1) for e in full[:2] for m in e]).astype(np.float16).view(np.uint8)
+    zero = np.zeros((D, D), dtype=np.float32)
+    token = np.arange(D)
+    inj = np.where(token[:, None] % 2 == np.arange(2)[None], 0.0, -1e4).astype(np.float32)
+    x = torch.eye(D, dtype=torch.float16, device="cuda")
+    for shared in (False, True):
+        parts = full[2] if shared else [zero] * 3
+        L = quant.LayerWeights(H=D, E=2, K=1, F=D, S=D, scaling=0.0 if shared else 1.0, router=np.zeros((2, D), np.uint16),
+                               expert_qtype=quant.QTYPE_F16, expert_qweight=slab, expert_qscale=None,
+                               **{n: quant.make_matrix(quant.QTYPE_F16, w) for n, w in zip(("shared_gate", "shared_up", "shared_down"), parts)})
+        g = Layer(pkg, L, D)
+        try:
+            out = torch.zeros((D, D), dtype=torch.float16, device="cuda")
+            g.ctx.layer_forward(0, x, D, out, injected_logits=dev(inj))
+            g.ctx.synchronize()
+        finally:
+            g.close()
+        w = np.stack([tests[2 if shared else k % 2][:, k] for k in token]).astype(np.float64)
+        got = out.cpu().numpy().astype(np.float64)
+        if hot == "gate":
+            want = w / (1 + np.exp(-w))
+            assert np.all(np.abs(got - want) <= 2.0 ** -10 * np.abs(want) + 2.0 ** -24), float(np.abs(got - want).max())
+        else:
+            assert np.array_equal(got, (64 * w if hot == "up" else w))
+
+
 @pytest.mark.parametrize("pad", [16, 48, 128 * 128 * 2])
 def test_fp16_slab_with_gaps_gives_the_packed_slabs_bits(pkg, pad):
     """Gaps of any multiple of 16 bytes between the projections: strides that are no multiples of one another, and ones that are

@@ -141,23 +141,13 @@ __device__ __forceinline__ void chunk_dot_f16(const uint4 &q, const float *x, in
     (void)xc;
 }
 
-// Lane-partial dot of one packed weight row with M activation rows (x: fp32 in shared memory,
-// row stride ld).  Caller reduces over the warp.
-template <int QT, int M>
-__device__ __forceinline__ void row_dot(const uint8_t *wrow, const __half *srow, uint32_t cols, const float *x, int ld,
-                                        int lane, float (&acc)[M]) {
-    const int chunks = (int)(cols / ChunkTraits<QT>::kWeights);
+// Lane-partial dot of one fp16 weight row with M activation rows (x: fp32 in shared memory, row stride ld).  Caller reduces
+// over the warp.
+template <int M>
+__device__ __forceinline__ void row_dot_f16(const __half *wrow, uint32_t cols, const float *x, int ld, int lane, float (&acc)[M]) {
+    const int chunks = (int)(cols / ChunkTraits<UOCR_QT_F16>::kWeights);
     const uint4 *w4 = reinterpret_cast<const uint4 *>(wrow);
-    for (int c = lane; c < chunks; c += 32) {
-        const uint4 q = __ldg(w4 + c);
-        if (QT == UOCR_QT_Q4) {
-            chunk_dot_q4<M>(q, x, ld, c, __half2float(srow[c >> 1]), acc);
-        } else if (QT == UOCR_QT_Q8) {
-            chunk_dot_q8<M>(q, x, ld, c, __half2float(srow[c >> 2]), acc);
-        } else {
-            chunk_dot_f16<M>(q, x, ld, c, acc);
-        }
-    }
+    for (int c = lane; c < chunks; c += 32) chunk_dot_f16<M>(__ldg(w4 + c), x, ld, c, acc);
 }
 
 __device__ __forceinline__ float silu_f32(float v) { return v / (1.0f + __expf(-v)); }

@@ -62,8 +62,7 @@ router_kernel(const __half *__restrict__ hidden, const __half *__restrict__ rout
             float acc[TPB];
 #pragma unroll
             for (int m = 0; m < TPB; ++m) acc[m] = 0.f;
-            row_dot<UOCR_QT_F16, TPB>(reinterpret_cast<const uint8_t *>(router + (size_t)e * H), nullptr, H, xs, (int)H,
-                                      lane, acc);
+            row_dot_f16<TPB>(router + (size_t)e * H, H, xs, (int)H, lane, acc);
 #pragma unroll
             for (int m = 0; m < TPB; ++m) {
                 const float v = warp_sum(acc[m]);

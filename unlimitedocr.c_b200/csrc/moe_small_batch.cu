@@ -127,11 +127,12 @@ __device__ __forceinline__ void stage_row(uint4 *stage, const uint8_t *wrow, int
 }
 __device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// (staged: how many of the row's pieces are in shared memory)
 template <int QT, int M>
-__device__ __forceinline__ void row_dot_staged(const uint4 *stage, const uint8_t *wrow, const __half *srow, uint32_t cols, const __half *x,
-                                               int lane, float *out) {
+__device__ __forceinline__ void row_dot_staged(const uint4 *stage, int staged, const uint8_t *wrow, const __half *srow, uint32_t cols,
+                                               const __half *x, int lane, float *out) {
     constexpr int kPerGroup = UOCR_GROUP / ChunkTraits<QT>::kWeights;
-    const int pieces = (int)(cols / ChunkTraits<QT>::kWeights), staged = staged_pieces(pieces);
+    const int pieces = (int)(cols / ChunkTraits<QT>::kWeights);
     float acc[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) acc[m] = 0.f;
@@ -175,9 +176,9 @@ gate_up_kernel(GroupSource src, const __half *__restrict__ hidden, uint32_t H, u
     const uint8_t *uw = gw + up_offset_bytes;
     const __half *gs = s_base ? s_base + rows.expert * expert_scale_stride + (size_t)row * groups : nullptr;
     const __half *us = s_base ? gs + up_scale_offset : nullptr;
-    const int pieces = (int)(H / ChunkTraits<QT>::kWeights);
-    uint4 *stage_g = reinterpret_cast<uint4 *>(xs + (size_t)kMaxM * H) + (size_t)warp * 2 * staged_pieces(pieces);
-    uint4 *stage_u = stage_g + staged_pieces(pieces);
+    const int pieces = (int)(H / ChunkTraits<QT>::kWeights), staged = staged_pieces(pieces);
+    uint4 *stage_g = reinterpret_cast<uint4 *>(xs + (size_t)kMaxM * H) + (size_t)warp * 2 * staged;
+    uint4 *stage_u = stage_g + staged;
     stage_row(stage_g, gw, pieces, lane);
     stage_row(stage_u, uw, pieces, lane);
 
@@ -193,15 +194,15 @@ gate_up_kernel(GroupSource src, const __half *__restrict__ hidden, uint32_t H, u
         if (i >= F) continue;
         float g[kMaxM], u[kMaxM];
         if (mc == 1) {
-            row_dot_staged<QT, 1>(stage_g, gw, gs, H, xs, lane, g);
-            row_dot_staged<QT, 1>(stage_u, uw, us, H, xs, lane, u);
+            row_dot_staged<QT, 1>(stage_g, staged, gw, gs, H, xs, lane, g);
+            row_dot_staged<QT, 1>(stage_u, staged, uw, us, H, xs, lane, u);
         } else if (mc == 2) {
-            row_dot_staged<QT, 2>(stage_g, gw, gs, H, xs, lane, g);
-            row_dot_staged<QT, 2>(stage_u, uw, us, H, xs, lane, u);
+            row_dot_staged<QT, 2>(stage_g, staged, gw, gs, H, xs, lane, g);
+            row_dot_staged<QT, 2>(stage_u, staged, uw, us, H, xs, lane, u);
         } else {
             // rows beyond mc read stale shared memory; their results are not stored
-            row_dot_staged<QT, kMaxM>(stage_g, gw, gs, H, xs, lane, g);
-            row_dot_staged<QT, kMaxM>(stage_u, uw, us, H, xs, lane, u);
+            row_dot_staged<QT, kMaxM>(stage_g, staged, gw, gs, H, xs, lane, g);
+            row_dot_staged<QT, kMaxM>(stage_u, staged, uw, us, H, xs, lane, u);
         }
         if (lane == 0) {
             for (uint32_t m = 0; m < mc; ++m) {
@@ -228,8 +229,8 @@ down_kernel(GroupSource src, const __half *__restrict__ mid, uint32_t H, uint32_
     const uint32_t wrow = min(h, H - 1u);
     const uint8_t *dw = w_base + rows.expert * expert_stride_bytes + (size_t)wrow * row_bytes;
     const __half *ds = s_base ? s_base + rows.expert * expert_scale_stride + (size_t)wrow * groups : nullptr;
-    const int pieces = (int)(F / ChunkTraits<QT>::kWeights);
-    uint4 *stage_d = reinterpret_cast<uint4 *>(xs + (size_t)kMaxM * F) + (size_t)warp * staged_pieces(pieces);
+    const int pieces = (int)(F / ChunkTraits<QT>::kWeights), staged = staged_pieces(pieces);
+    uint4 *stage_d = reinterpret_cast<uint4 *>(xs + (size_t)kMaxM * F) + (size_t)warp * staged;
     stage_row(stage_d, dw, pieces, lane);
 
     for (uint32_t r0 = 0; r0 < rows.count; r0 += kMaxM) {
@@ -243,9 +244,9 @@ down_kernel(GroupSource src, const __half *__restrict__ mid, uint32_t H, uint32_
         __syncthreads();
         if (h >= H) continue;
         float acc[kMaxM];
-        if (mc == 1) row_dot_staged<QT, 1>(stage_d, dw, ds, F, xs, lane, acc);
-        else if (mc == 2) row_dot_staged<QT, 2>(stage_d, dw, ds, F, xs, lane, acc);
-        else row_dot_staged<QT, kMaxM>(stage_d, dw, ds, F, xs, lane, acc);
+        if (mc == 1) row_dot_staged<QT, 1>(stage_d, staged, dw, ds, F, xs, lane, acc);
+        else if (mc == 2) row_dot_staged<QT, 2>(stage_d, staged, dw, ds, F, xs, lane, acc);
+        else row_dot_staged<QT, kMaxM>(stage_d, staged, dw, ds, F, xs, lane, acc);
         if (lane == 0)
             for (uint32_t m = 0; m < mc; ++m) {
                 const uint32_t row = rows.pairs ? rows.pairs[r0 + m] : (r0 + m);
@@ -795,37 +796,42 @@ cudaError_t launch_lm_head_argmax(const DMatrix &m, const __half *hidden, uint32
 }
 
 // ---- dequantisation probe ------------------------------------------------------------------------------------
-// out[row][col] = the f32 value the matrix-vector kernels give weight (row, col): the row is multiplied, through the
-// same row_dot() the layer kernels use, with a one-hot activation vector per column, which leaves level * scale.
-// One CTA per row, one activation buffer per warp.
+// out[row][col] = the f32 value the matrix-vector kernels give weight (row, col): the row is staged and multiplied as the
+// layer kernels do it (stage_row, row_dot_staged) with two activation rows, of which one is one-hot and the other zero; the
+// two results add up to level * scale.  Odd rows are read with their first half of pieces staged and the rest from global
+// memory.  One CTA per row, one staged row and one pair of activation rows per warp.
 constexpr int kProbeWarps = 4;
 
 template <int QT>
 __global__ void __launch_bounds__(kProbeWarps * 32)
 dequant_probe_kernel(const uint8_t *__restrict__ w, const __half *__restrict__ s, uint32_t cols, uint32_t row_bytes,
                      float *__restrict__ out) {
-    extern __shared__ float xs[];   // [kProbeWarps][cols]
+    extern __shared__ __align__(16) __half probe_xs[];   // [kProbeWarps][2][cols], then the warps' staged rows
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t row = blockIdx.x, groups = cols / UOCR_GROUP;
-    float *x = xs + (size_t)warp * cols;
-    for (uint32_t c = lane; c < cols; c += 32) x[c] = 0.f;
-    __syncwarp();
+    const int pieces = (int)(cols / ChunkTraits<QT>::kWeights), staged = staged_pieces(pieces);
+    __half *x = probe_xs + (size_t)warp * 2 * cols;
+    uint4 *stage = reinterpret_cast<uint4 *>(probe_xs + (size_t)kProbeWarps * 2 * cols) + (size_t)warp * staged;
     const uint8_t *wrow = w + (size_t)row * row_bytes;
     const __half *srow = s ? s + (size_t)row * groups : nullptr;
+    stage_row(stage, wrow, pieces, lane);
+    for (uint32_t c = lane; c < 2 * cols; c += 32) x[c] = __ushort_as_half(0);
+    stage_wait();
+    __syncwarp();
     for (uint32_t c = warp; c < cols; c += kProbeWarps) {
-        if (lane == 0) x[c] = 1.f;
+        __half *hot = x + (c / kProbeWarps & 1u) * cols + c;
+        if (lane == 0) *hot = __float2half_rn(1.f);
         __syncwarp();
-        float acc[1] = {0.f};
-        row_dot<QT, 1>(wrow, srow, cols, x, (int)cols, lane, acc);
-        const float v = warp_sum(acc[0]);
-        if (lane == 0) { out[(size_t)row * cols + c] = v; x[c] = 0.f; }
+        float v[2];
+        row_dot_staged<QT, 2>(stage, row & 1u ? staged / 2 : staged, wrow, srow, cols, x, lane, v);
+        if (lane == 0) { out[(size_t)row * cols + c] = v[0] + v[1]; *hot = __ushort_as_half(0); }
         __syncwarp();
     }
 }
 
 cudaError_t launch_dequant_probe(const DMatrix &m, float *out, cudaStream_t st, uint64_t *launches) {
-    const size_t smem = sizeof(float) * kProbeWarps * m.cols;
-    if (smem > 48 * 1024) return cudaErrorInvalidValue;
+    if (m.cols > 2048) return cudaErrorInvalidValue;      // 48 KB: 4 warps x (2 x 4 KB of activations + 4 KB of weights)
+    const size_t smem = kProbeWarps * (2 * sizeof(__half) * m.cols + 16 * (size_t)kStagePieces);
     UOCR_QT_SWITCH(m.qtype, (dequant_probe_kernel<QT><<<m.rows, kProbeWarps * 32, smem, st>>>(m.w, m.s, m.cols, m.row_bytes, out)));
     ++*launches;
     return cudaGetLastError();

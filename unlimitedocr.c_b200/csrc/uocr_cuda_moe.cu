@@ -73,7 +73,7 @@ cudaError_t launch_batched_experts(const DLayer &L, const Scratch &S, uint32_t n
 cudaError_t launch_batched_combine(const DLayer &L, const Scratch &S, const __half *residual, uint32_t n, uint8_t *scratch, __half *out,
                                    cudaStream_t st, uint64_t *launches);
 cudaError_t launch_dequant_probe(const DMatrix &m, float *out, cudaStream_t st, uint64_t *launches);
-cudaError_t launch_producer_probe(const DMatrix &m, float *out, cudaStream_t st, uint64_t *launches);
+cudaError_t launch_producer_probe(const DMatrix &m, float *out, uint32_t *status, cudaStream_t st, uint64_t *launches);
 int decode_grid_size();
 bool decode_supported(const DLayer *layers, uint32_t first, uint32_t count);
 bool decode_sliced_layer_ok(const DLayer &L);
@@ -1049,8 +1049,8 @@ extern "C" int uocr_cuda_moe_debug_dequantize(uocr_cuda_context *ctx, uint32_t l
         return fail(ctx, error, error_size, "matrix selector %u out of range (0-2 routed gate/up/down, 3-5 shared)", matrix);
     }
     if (path == 0) CU_TRY(ctx, uocr::launch_dequant_probe(m, d_out, ctx->stream, &ctx->launches));
-    else if (path == 1) CU_TRY(ctx, uocr::launch_producer_probe(m, d_out, ctx->stream, &ctx->launches));
-    else return fail(ctx, error, error_size, "path selector %u out of range (0 matrix-vector kernels, 1 tensor-core producer)", path);
+    else if (path == 1) CU_TRY(ctx, uocr::launch_producer_probe(m, d_out, ctx->status, ctx->stream, &ctx->launches));
+    else return fail(ctx, error, error_size, "path selector %u out of range (0 matrix-vector kernels, 1 tensor-core operand)", path);
     return 1;
 }
 
