@@ -320,8 +320,8 @@ UOCR_CUDA_API int uocr_cuda_moe_dispatch_plan(uocr_cuda_context *ctx, const uint
  * this with uocr_alloc_guard, src/core/uocr_alloc.h:21-42), in a decode loop that has frozen its
  * memory map, or after the engine's memory admission has handed out the whole device budget.
  * Limits: n_experts <= 256 and n_tokens * top_k <= 1048576; larger sizes are refused with a message.
- * The first call on a device looks up the array's device address and raises the kernel's shared-memory limit
- * (no allocation); make that first call before any stream capture.  All calls share the one array, so two calls
+ * The first call on a device looks up the array's device address (no allocation); make that first call before any
+ * stream capture.  All calls share the one array, so two calls
  * whose kernels may overlap on the GPU (different streams without an ordering between them) race on it; calls
  * on one stream are safe.  Nothing in the array needs clearing: every call rewrites the entries it later reads.
  * cuda_stream is a cudaStream_t (NULL = the default stream); the current device is used. */

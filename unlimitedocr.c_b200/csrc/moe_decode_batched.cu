@@ -6,7 +6,7 @@
 //    once), the exact softmax / top-k, and the token's activations rewritten as block-floating-point bytes (two
 //    signed bytes per value, one scale per 64-wide group) - the B operand of the integer MMAs, computed once per
 //    token instead of once per expert that uses it.  The CTA that finishes last builds the dispatch plan (a stable
-//    counting sort of the at most 384 pairs).
+//    counting sort of the at most 1024 pairs).
 // 2. decode_batched_kernel, weight-stationary on the slice-major "unit blobs" of the single-token decode kernel.  A
 //    work item is (expert, 16-token pass, one or two consecutive 64-wide slices of the intermediate dimension); the shared
 //    MLP counts as two more experts that every token selects.  Items are listed hottest expert first and dealt
@@ -37,7 +37,7 @@ constexpr int kBtThreads = kBtConsumers + 64;                  // + a warp that 
 constexpr int kBtTokens = 16;                                  // tokens per pass
 // An item covers SLICES consecutive 64-wide slices of its expert (template parameter of the kernel): two for calls of more
 // than 16 tokens (7 parts per expert and pass), one for smaller calls (14 parts), whose ~150 two-slice items would leave most
-// CTAs idle during a second wave.  The partial-output buffers are sized for 14 parts.
+// CTAs idle during a second wave.
 constexpr int kBtSmallCallTokens = 16;
 __host__ __device__ constexpr int bt_slices_for(uint32_t n) { return n <= (uint32_t)kBtSmallCallTokens ? 1 : 2; }
 constexpr int kBtSharedHalves = kSlS / 64 / kSlRoutedPerSlot;  // the shared MLP as 2 pseudo-experts of 14 slices
@@ -66,7 +66,7 @@ struct RouteSmallParams {
     float *weights;                 // [n][K]
     uint32_t *x_limbs;              // [n][20][2][16 words]
     float *x_scales;                // [n][20]
-    uint32_t *offsets, *pair_rows, *inverse, *active;      // the dispatch plan
+    uint32_t *offsets, *pair_rows, *inverse;      // the dispatch plan
     uint32_t *ticket;               // zero between launches
     uint32_t *status;
     unsigned long long *acc;        // [n][H] fixed-point output sums of the call: this kernel clears its token's row
@@ -169,25 +169,22 @@ __global__ void __launch_bounds__(kRsThreads) route_small_kernel(const RouteSmal
     if (lane < 4) s_cnt[4 * warp + lane] = lane == 0 ? cnt[0] : lane == 1 ? cnt[1] : lane == 2 ? cnt[2] : cnt[3];
     __syncthreads();
     if (warp == 0) {
-        // exclusive prefix sums of the 64 counts and of the "has pairs" flags: lane l takes experts 2l and 2l + 1
+        // exclusive prefix sums of the 64 counts: lane l takes experts 2l and 2l + 1
         const uint32_t c0 = s_cnt[2 * lane], c1 = s_cnt[2 * lane + 1];
-        uint32_t sum = c0 + c1, act = (c0 ? 1u : 0u) + (c1 ? 1u : 0u);
+        uint32_t sum = c0 + c1;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t s2 = __shfl_up_sync(0xffffffffu, sum, o), a2 = __shfl_up_sync(0xffffffffu, act, o);
-            if (lane >= o) { sum += s2; act += a2; }
+            const uint32_t s2 = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += s2;
         }
-        const uint32_t base = sum - c0 - c1, abase = act - (c0 ? 1u : 0u) - (c1 ? 1u : 0u);
+        const uint32_t base = sum - c0 - c1;
         prm.offsets[2 * lane] = base;
         prm.offsets[2 * lane + 1] = base + c0;
-        if (c0) prm.active[1 + abase] = (uint32_t)(2 * lane);
-        if (c1) prm.active[1 + abase + (c0 ? 1u : 0u)] = (uint32_t)(2 * lane + 1);
         __syncwarp();
         s_cnt[2 * lane] = base;
         s_cnt[2 * lane + 1] = base + c0;
         if (lane == 31) {
             prm.offsets[E] = sum;
-            prm.active[0] = act;
             *prm.ticket = 0u;
         }
     }
@@ -633,13 +630,12 @@ static std::atomic<int> g_bt_sms[64];
 
 uint32_t decode_batched_max_tokens() { return kBtMaxTokens; }
 
-// Scratch of a call with n tokens (n <= decode_batched_max_tokens()): the parts of the routed experts and of the shared
-// MLP, the tokens' activation bytes and scales.
-BatchedScratchLayout decode_batched_scratch(uint32_t n, uint32_t K) {
+// Scratch of a call with n tokens (n <= decode_batched_max_tokens()): the output sums, the tokens' activation bytes and
+// scales.
+BatchedScratchLayout decode_batched_scratch(uint32_t n) {
     BatchedScratchLayout l{};
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off = (off + bytes + 255) / 256 * 256; return o; };
-    (void)K;
     l.acc = take((size_t)n * kSlH * sizeof(unsigned long long));
     l.x_limbs = take((size_t)n * kBtTokenLimbBytes);
     l.x_scales = take((size_t)n * kSlGroups * sizeof(float));
@@ -653,17 +649,17 @@ bool decode_batched_supported(const DLayer &L, uint32_t n) {
 }
 
 // The layer for n tokens in three launches: routing + activation bytes + dispatch plan (results in S), experts, combine.
-// scratch: a region of decode_batched_scratch(n, K).total bytes; ticket: a word that is zero before the first call
+// scratch: a region of decode_batched_scratch(n).total bytes; ticket: a word that is zero before the first call
 // (every call leaves it zero).
 cudaError_t launch_batched_route(const DLayer &L, const Scratch &S, const __half *hidden, const float *injected, uint32_t n,
                                  float *logits, float *probs, uint8_t *scratch, uint32_t *ticket, cudaStream_t st, uint64_t *launches,
                                  const __half *norm_weight, float norm_eps) {
-    const BatchedScratchLayout lay = decode_batched_scratch(n, L.K);
+    const BatchedScratchLayout lay = decode_batched_scratch(n);
     RouteSmallParams r{};
     r.hidden = hidden; r.norm_weight = norm_weight; r.norm_eps = norm_eps; r.router = L.router; r.bias = L.bias; r.injected = injected; r.n = n; r.K = L.K; r.scaling = L.scaling;
     r.logits_out = logits; r.probs_out = probs; r.ids = S.top_ids; r.weights = S.top_weights;
     r.x_limbs = reinterpret_cast<uint32_t *>(scratch + lay.x_limbs); r.x_scales = reinterpret_cast<float *>(scratch + lay.x_scales);
-    r.offsets = S.expert_offsets; r.pair_rows = S.pair_rows; r.inverse = S.inverse; r.active = S.active;
+    r.offsets = S.expert_offsets; r.pair_rows = S.pair_rows; r.inverse = S.inverse;
     r.ticket = ticket; r.status = S.status;
     r.acc = reinterpret_cast<unsigned long long *>(scratch + lay.acc);
     if (L.expert_qtype == UOCR_QT_Q4) route_small_kernel<UOCR_QT_Q4><<<n, kRsThreads, 0, st>>>(r);
@@ -681,7 +677,7 @@ cudaError_t launch_batched_experts(const DLayer &L, const Scratch &S, uint32_t n
         if ((err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return err;
         if (dev >= 0 && dev < 64) g_bt_sms[dev] = sms;
     }
-    const BatchedScratchLayout lay = decode_batched_scratch(n, L.K);
+    const BatchedScratchLayout lay = decode_batched_scratch(n);
     BatchedParams p{};
     p.units = L.dec_units;
     p.x_limbs = reinterpret_cast<const uint32_t *>(scratch + lay.x_limbs); p.x_scales = reinterpret_cast<const float *>(scratch + lay.x_scales);
@@ -710,7 +706,7 @@ cudaError_t launch_batched_experts(const DLayer &L, const Scratch &S, uint32_t n
 cudaError_t launch_batched_combine(const DLayer &L, const Scratch &S, const __half *residual, uint32_t n, uint8_t *scratch, __half *out,
                                    cudaStream_t st, uint64_t *launches) {
     (void)S;
-    const BatchedScratchLayout lay = decode_batched_scratch(n, L.K);
+    const BatchedScratchLayout lay = decode_batched_scratch(n);
     const size_t work = (size_t)n * (L.H / 4);
     finalize_batched_kernel<<<(unsigned)((work + 255) / 256), 256, 0, st>>>(reinterpret_cast<const unsigned long long *>(scratch + lay.acc), residual, n,
                                                                             L.H, out);

@@ -144,11 +144,15 @@ __device__ __forceinline__ void row_dot_staged(const uint4 *stage, int staged, c
 #pragma unroll
     for (int m = 0; m < M; ++m) out[m] = warp_sum(acc[m]);
 }
+// Shared memory of a launch: kMaxM activation rows, and the staged weight rows of every warp (gate/up two, down one)
 template <int QT>
-static size_t gemv_smem(uint32_t cols, uint32_t rows_per_warp) {
+static constexpr size_t gemv_smem(uint32_t cols, uint32_t rows_per_warp) {
     const uint32_t pieces = cols / ChunkTraits<QT>::kWeights;
     return (size_t)kMaxM * cols * sizeof(__half) + (size_t)(pieces < (uint32_t)kStagePieces ? pieces : kStagePieces) * 16 * rows_per_warp * kGemvWarps;
 }
+// the widest rows the kernels take: hidden, and the dense MLP's intermediate width
+constexpr uint32_t kGateUpMaxCols = 3072, kDownMaxCols = 8192;
+static bool gemv_fits(uint32_t hidden, uint32_t inner) { return hidden <= kGateUpMaxCols && inner <= kDownMaxCols; }
 // one row of fp16 activations into shared memory (cols: a multiple of 64; a caller's own rows may start at any even address)
 __device__ __forceinline__ void stage_activations(__half *xs, const __half *row, uint32_t cols) {
     if (reinterpret_cast<uintptr_t>(row) & 15u) {
@@ -275,8 +279,6 @@ __global__ void combine_kernel(const float *__restrict__ down_out, const float *
     out[idx] = __float2half_rn(acc);
 }
 
-constexpr int kDenseSmemBytes = 4 * 8192 * (int)sizeof(float);
-
 template <int QT>
 static void launch_gate_up(const GroupSource &src, uint32_t n_groups, const __half *hidden, uint32_t H, uint32_t F,
                            const uint8_t *w, const __half *s, uint64_t stride, uint64_t up_off, uint64_t sstride,
@@ -307,12 +309,12 @@ static uint32_t packed_row_bytes(int qt, uint32_t cols) {
 }
 
 cudaError_t init_small_batch_kernels() {
-    // activations of four tokens in fp16 (gate/up: up to 3072 wide, down: the dense MLP's intermediate width, up to 8192) and
-    // the staged weight rows of eight warps (two rows each for gate/up), 4 KB a row at most
     cudaError_t err = cudaSuccess;
-#define UOCR_GEMV_SMEM(QT)                                                                                                           \
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(gate_up_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 88 * 1024); \
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(down_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+#define UOCR_GEMV_SMEM(QT)                                                                                              \
+    if (err == cudaSuccess)                                                                                             \
+        err = cudaFuncSetAttribute(gate_up_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemv_smem<QT>(kGateUpMaxCols, 2)); \
+    if (err == cudaSuccess)                                                                                             \
+        err = cudaFuncSetAttribute(down_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemv_smem<QT>(kDownMaxCols, 1));
     UOCR_GEMV_SMEM(UOCR_QT_Q4) UOCR_GEMV_SMEM(UOCR_QT_Q8) UOCR_GEMV_SMEM(UOCR_QT_F16)
 #undef UOCR_GEMV_SMEM
     return err;
@@ -321,9 +323,7 @@ cudaError_t init_small_batch_kernels() {
 // ---- dense SwiGLU MLP (the first decoder layer's MLP; uocr_cpu_ref_dense_swiglu_f32, src/backend/cpu_ref/uocr_cpu_ref.c:305-349) ----
 // A few tokens through gate/up, down and the residual add with the kernels the shared experts use:
 // out = fp16( down . fp16(silu(gate x) * up x) + residual ), f32 sums, one rounding of the result.
-bool dense_small_supported(uint32_t H, uint32_t S) {
-    return (size_t)kMaxM * H * sizeof(float) <= 48 * 1024 && (size_t)kMaxM * S * sizeof(float) <= (size_t)kDenseSmemBytes;
-}
+bool dense_small_supported(uint32_t H, uint32_t S) { return gemv_fits(H, S); }
 
 cudaError_t launch_dense_small(const DMatrix &g, const DMatrix &u, const DMatrix &d, const __half *hidden, const __half *residual,
                                uint32_t n, __half *mid, float *out_f32, __half *out, cudaStream_t st, uint64_t *launches) {
@@ -345,7 +345,7 @@ cudaError_t launch_dense_small(const DMatrix &g, const DMatrix &u, const DMatrix
 cudaError_t launch_small_batch_layer(const DLayer &L, const Scratch &S, const __half *hidden, const __half *residual,
                                      uint32_t n, __half *out, cudaStream_t st, uint64_t *launches) {
     const uint32_t H = L.H, F = L.F, Sd = L.S, K = L.K, E = L.E;
-    if ((size_t)kMaxM * (H > Sd ? H : Sd) * sizeof(float) > 48 * 1024) return cudaErrorInvalidValue;
+    if (!gemv_fits(H, F > Sd ? F : Sd)) return cudaErrorInvalidValue;
     GroupSource routed{S.active, S.expert_offsets, S.pair_rows, n, K};
     GroupSource shared{nullptr, nullptr, nullptr, n, K};
     const uint32_t max_groups = (uint64_t)n * K < E ? n * K : E;

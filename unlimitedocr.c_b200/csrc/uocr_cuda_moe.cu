@@ -64,7 +64,7 @@ cudaError_t launch_gemm_combine(const DLayer &L, const Scratch &S, const GemmScr
                                 const __half *residual, uint32_t n, __half *out, cudaStream_t st, uint64_t *launches);
 cudaError_t init_decode_batched_kernels();
 uint32_t decode_batched_max_tokens();
-BatchedScratchLayout decode_batched_scratch(uint32_t n, uint32_t K);
+BatchedScratchLayout decode_batched_scratch(uint32_t n);
 bool decode_batched_supported(const DLayer &L, uint32_t n);
 cudaError_t launch_batched_route(const DLayer &L, const Scratch &S, const __half *hidden, const float *injected, uint32_t n,
                                  float *logits, float *probs, uint8_t *scratch, uint32_t *ticket, cudaStream_t st, uint64_t *launches,
@@ -906,7 +906,7 @@ static ArenaLayout layout_arena(uint32_t H, uint32_t E, uint32_t K, uint32_t F, 
     }
     {   // batched decode path (calls of up to 64 tokens): the call's fixed-point output sums, the tokens' activation bytes
         const uint32_t nb = n < uocr::decode_batched_max_tokens() ? n : uocr::decode_batched_max_tokens();
-        a.bt_routed = take(uocr::decode_batched_scratch(nb, K).total);
+        a.bt_routed = take(uocr::decode_batched_scratch(nb).total);
     }
     a.total = off;
     return a;
