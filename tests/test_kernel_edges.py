@@ -85,27 +85,45 @@ def test_fp16_slab_with_gaps_gives_the_packed_slabs_bits(pkg, pad):
     assert all(torch.equal(a, b) for a, b in zip(outs[:3], outs[3:]))
 
 
-@pytest.mark.parametrize("n,K,E", [(31, 1, 8), (341, 3, 9), (512, 2, 8), (205, 5, 10), (1025, 1, 256), (1365, 6, 64), (1366, 6, 64)])
+@pytest.mark.parametrize("n,K,E", [(31, 1, 8), (341, 3, 9), (512, 2, 8), (205, 5, 10), (1025, 1, 256), (1365, 6, 64), (1366, 6, 64),
+                                   (1366, 6, 63), (1366, 6, 130)])
 def test_dispatch_plan_at_step_edges(pkg, n, K, E):
-    """Pair counts around a warp's step, a CTA's round and the limit of the one-CTA plan; some experts without pairs, some ids
-    out of range."""
+    """Pair counts around a warp's step and a CTA's round, and around the 8192 pairs above which a context's plan takes the
+    many-CTA form (for an even E up to 128); some experts without pairs, some ids out of range.  Both entry points: the
+    allocation-free one always runs the one-CTA form."""
     rng = np.random.default_rng(n)
     ids = rng.integers(0, max(1, E - 2), size=(n, K)).astype(np.uint32)
     ids[rng.integers(0, n, 3), 0] = E + 1
-    off = torch.zeros(E + 1, dtype=torch.int32).cuda()
-    rows = torch.full((n * K,), -1, dtype=torch.int32).cuda()
-    inv = torch.zeros(n * K, dtype=torch.int32).cuda()
-    pkg.ffi.dispatch_plan_noalloc(dev(ids.view(np.int32)), n, K, E, off, rows, inv)
-    torch.cuda.synchronize()
     flat = ids.reshape(-1)
     order = np.argsort(flat, kind="stable")
     order = order[flat[order] < E]
     want_inv = np.full(n * K, 0xFFFFFFFF, dtype=np.uint32)
     want_inv[order] = np.arange(order.size, dtype=np.uint32)
     counts = np.bincount(flat[flat < E], minlength=E)
-    assert np.array_equal(off.cpu().numpy(), np.concatenate([[0], np.cumsum(counts)]))
-    assert np.array_equal(rows.cpu().numpy()[: order.size], order)
-    assert np.array_equal(inv.cpu().numpy().view(np.uint32), want_inv)
+    L, _, _ = make(1, dict(H=64, E=E, K=K, F=64, S=64), "q8_0", 1)
+    g = Layer(pkg, L, n)
+    try:
+        for plan in (pkg.ffi.dispatch_plan_noalloc, g.ctx.dispatch_plan):
+            off = torch.zeros(E + 1, dtype=torch.int32).cuda()
+            rows = torch.full((n * K,), -1, dtype=torch.int32).cuda()
+            inv = torch.zeros(n * K, dtype=torch.int32).cuda()
+            before = g.ctx.kernel_launches
+            plan(dev(ids.view(np.int32)), n, K, E, off, rows, inv)
+            torch.cuda.synchronize()
+            if plan == g.ctx.dispatch_plan:
+                assert g.ctx.kernel_launches - before == (3 if n * K > 8192 and E % 2 == 0 and E <= 128 else 1)
+            assert np.array_equal(off.cpu().numpy(), np.concatenate([[0], np.cumsum(counts)]))
+            assert np.array_equal(rows.cpu().numpy()[: order.size], order)
+            assert np.array_equal(inv.cpu().numpy().view(np.uint32), want_inv)
+    finally:
+        g.close()
+
+
+@pytest.mark.parametrize("n,E", [(1365, 64), (1366, 64), (1366, 63), (1366, 130)])
+def test_grouped_gemm_with_tile_lists_of_either_plan(pkg, port, n, E):
+    """Tile lists written by the one-CTA plan (up to 8192 pairs, or an odd E, or E above 128) and by the many-CTA one."""
+    L, hidden, resid = make(800 + E, dict(H=128, E=E, K=6, F=128, S=128), "q8_0", n, bias="zipf")
+    check_layer(pkg, port, L, hidden, resid, gemm=True)
 
 
 @pytest.mark.parametrize("qname", ["q4_0", "q8_0"])
