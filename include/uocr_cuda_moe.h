@@ -154,7 +154,8 @@ UOCR_CUDA_API uint64_t uocr_cuda_context_moe_scratch_bytes(const uocr_cuda_conte
 
 /* ---- model mapping: counterpart of uocr_metal_context_map_model / _unmap_model
  * (src/backend/metal/uocr_metal.h:178-181).  Metal wraps the mmap'd file without a copy;
- * here every tensor of the layer is validated and uploaded once.  desc holds HOST pointers.
+ * here every tensor of the layer is validated and uploaded once (an fp16 slab with gaps is packed on the way).  desc
+ * holds HOST pointers.
  * Layers get consecutive indices starting at 0. */
 UOCR_CUDA_API int uocr_cuda_context_map_moe_layer(uocr_cuda_context *ctx, const uocr_cuda_moe_layer_desc *h_desc,
                                                   uint32_t *out_layer_index, char *error, size_t error_size);
